@@ -22,8 +22,10 @@
 #include <cfloat>
 #include <cmath>
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include "../../include/amigo_b200.h"
@@ -535,6 +537,27 @@ __device__ __forceinline__ PivotChoice choose_pivot(bool root, int k, int nc,
     }
   }
   return p;
+}
+
+// Whether choose_pivot takes the candidate itself as a 1x1 pivot at once
+// (colmax: the largest |entry| below the diagonal; a root front has candidate
+// rows only).
+__device__ __forceinline__ bool plain_pivot(bool root, double wkk, double colmax,
+                                            double ustab, double pivot_tol) {
+  const double bk_alpha = (1.0 + sqrt(17.0)) / 8.0;
+  const double abswkk = fabs(wkk);
+  return root ? abswkk > 0.0 && abswkk >= bk_alpha * colmax
+              : abswkk >= pivot_tol && abswkk >= ustab * colmax;
+}
+
+// Whether choose_pivot needs column imax.
+__device__ __forceinline__ bool needs_imax(bool root, int k, int nc, double wkk,
+                                           double abswik, double ctail, double ustab,
+                                           double pivot_tol) {
+  const double bk_alpha = (1.0 + sqrt(17.0)) / 8.0;
+  const double abswkk = fabs(wkk);
+  if (root) return fmax(abswkk, abswik) > 0.0 && !(abswkk >= bk_alpha * abswik);
+  return !(abswkk >= pivot_tol && abswkk >= ustab * fmax(abswik, ctail)) && k + 1 < nc;
 }
 
 // W[r, col] = src(r) - F[r, kstart:kstart+kw] . ctl.wrow  for r in [k, n),
@@ -1328,7 +1351,7 @@ k_big_setup(DevicePlan d, const int* __restrict__ nodes) {
 }
 
 __device__ __forceinline__ bool big_skip(const DevicePlan& d) {
-  return (*((volatile int*)d.status) & (ST_POOL_F | ST_POOL_I)) != 0;
+  return (*((volatile int*)d.status) & (ST_POOL_F | ST_POOL_I | ST_WAIT)) != 0;
 }
 
 template <class T>
@@ -2636,6 +2659,8 @@ k_big_panel_cl(DevicePlan d, const int* __restrict__ nodes, double ustab,
   }
 }
 
+#include "panel_rows.cuh"
+
 template <class T>
 __global__ void __launch_bounds__(NT, 2)
 k_big_update(DevicePlan d, const int* __restrict__ nodes) {
@@ -2711,7 +2736,7 @@ k_big_finalize(DevicePlan d, const int* __restrict__ nodes) {
 
 // Number of large fronts of the level still holding candidates; 0 when a
 // pool ran out (the fronts stopped and the host grows the pool and
-// restarts the factorization).
+// restarts the factorization) or a wait did (the host returns the error).
 __global__ void k_big_remaining(DevicePlan d, const int* __restrict__ nodes,
                                 int count, int* out) {
   int r = 0;
@@ -2766,8 +2791,9 @@ static int sm_count() {
   return n;
 }
 
-// Whether clusters of 16 CTAs of the global-scratch panel can be scheduled
-// on this device (set once, with the kernels' attributes).
+// Whether clusters of 16 CTAs of the row-per-thread panel and of the
+// global-scratch panel can be scheduled on this device (set once, with the
+// kernels' attributes).
 template <class T>
 static bool& cl16_ok() {
   static bool ok = false;
@@ -2804,6 +2830,69 @@ static int launch_panel_cl(int fronts, int smem, cudaStream_t s, const DevicePla
                              nodes, ustab, pivot_tol, smem, width_rule, fit_rows,
                              (int*)nullptr, scratch, stride));
   return 0;
+}
+
+// Shared memory of k_big_panel_rows for the most rows a launch takes.
+template <class T, int RPT, int CS>
+static int rows_attributes() {
+  auto kernel = k_big_panel_rows<T, kRowThreads, RPT, CS>;
+  const int rows = CS * kRowThreads * RPT;
+  FCUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)row_smem<T>(cl_local_rows<CS>(rows) + 1, rows)));
+  if (CS > 8)
+    FCUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  return 0;
+}
+
+// One panel of the level's fronts on k_big_panel_rows (PT threads a CTA, RPT
+// rows a thread, clusters of CS CTAs).
+template <class T, int RPT, int CS>
+static int launch_rows_at(int device, int fronts, cudaStream_t s, const DevicePlan& d,
+                          const int* nodes, double ustab, double pivot_tol, int rows) {
+  auto kernel = k_big_panel_rows<T, kRowThreads, RPT, CS>;
+  const int lld = cl_local_rows<CS>(rows) + 1;
+  const size_t smem = row_smem<T>(lld, rows);
+  // the kernel's attributes, once per device (always the same values, so
+  // threads that meet here do no harm)
+  static std::atomic<unsigned long long> set{0};
+  if (!(set.load() >> (device & 63) & 1)) {
+    const int rc = rows_attributes<T, RPT, CS>();
+    if (rc) return rc;
+    set.fetch_or(1ull << (device & 63));
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(fronts * CS);
+  cfg.blockDim = dim3(kRowThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CS;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CS > 1 ? 2 : 1;
+  FCUDA(cudaLaunchKernelEx(&cfg, kernel, d, nodes, ustab, pivot_tol, lld, rows, rows));
+  return 0;
+}
+
+template <class T>
+static int launch_panel_rows(int device, int fronts, cudaStream_t s,
+                             const DevicePlan& d, const int* nodes, double ustab, double pivot_tol, int rows) {
+  constexpr int PT = kRowThreads;
+  if (rows <= PT)
+    return launch_rows_at<T, 1, 1>(device, fronts, s, d, nodes, ustab, pivot_tol, rows);
+  if (rows <= 2 * PT)
+    return launch_rows_at<T, 1, 2>(device, fronts, s, d, nodes, ustab, pivot_tol, rows);
+  if (rows <= 4 * PT)
+    return launch_rows_at<T, 1, 4>(device, fronts, s, d, nodes, ustab, pivot_tol, rows);
+  if (rows <= 8 * PT)
+    return launch_rows_at<T, 1, 8>(device, fronts, s, d, nodes, ustab, pivot_tol, rows);
+  if (rows <= 16 * PT)
+    return launch_rows_at<T, 1, 16>(device, fronts, s, d, nodes, ustab, pivot_tol, rows);
+  return launch_rows_at<T, 2, 16>(device, fronts, s, d, nodes, ustab, pivot_tol, rows);
 }
 
 template <class T>
@@ -2858,6 +2947,15 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
               &nclu, k_big_panel_cl<T, kClThreads, kClRowsG, 16, false, true>, &q) !=
           cudaSuccess)
         nclu = 0;
+      // the row-per-thread panel on clusters of 16 at its largest
+      if (nclu > 0) {
+        const int rc = rows_attributes<T, 2, 16>();
+        if (rc) return rc;
+        q.dynamicSmemBytes = row_smem<T>(2 * kRowThreads + 1, 32 * kRowThreads);
+        if (cudaOccupancyMaxActiveClusters(&nclu, k_big_panel_rows<T, kRowThreads, 2, 16>,
+                                           &q) != cudaSuccess)
+          nclu = 0;
+      }
       cudaGetLastError();
       cl16_ok<T>() = nclu > 0;
     }
@@ -2926,22 +3024,24 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       // shared-W panel for levels whose fronts fit its rows; its shared
       // memory holds up to NB columns of W for the largest static front
       // (fronts grown by delayed pivots get fewer columns)
-      // cluster panel for levels of large fronts (mode 0: full-width
-      // panels; mode 2: the one-CTA panel's widths); its shared memory
-      // holds NB columns of W for kClSlack rows more than the largest
-      // static front
-      const bool use_cl = (h.panel_mode == 0 || h.panel_mode == 2) && fm >= h.cl_min_rows &&
+      // the row-per-thread panel (mode 0), for kClSlack rows more than the
+      // largest static front; in mode 2 the shared-memory cluster panel with
+      // the one-CTA panel's widths
+      const int row_rows = (int)fm + kClSlack;
+      const bool use_rows = h.panel_mode == 0 && fm >= h.cl_min_rows &&
+                            row_rows <= (cl16_ok<T>() ? 32 : 8) * kRowThreads;
+      const bool use_cl = h.panel_mode == 2 && fm >= h.cl_min_rows &&
                           fm + kClSlack <= kClMaxRows;
       const int cl_rule = h.panel_mode == 2 ? 1 : 0;
       const int cl_smem =
           use_cl ? 2 * NB * cl_local_rows<kClCS>((int)fm + kClSlack) * (int)sizeof(T) : 0;
-      // past shared memory: the cluster panel with its W and L rows in a
-      // global scratch region (clusters of 8, or 16 for the largest fronts;
-      // mode 3, a test mode: clusters of 16 on every level they can take,
+      // past its rows: the cluster panel with its W and L rows in a global
+      // scratch region (clusters of 8, or 16 for the largest fronts; mode 3,
+      // a test mode: clusters of 16 on every level they can take,
       // bit-identical to mode 0)
       const long long gmax = cl16_ok<T>() ? kClMaxRowsG16 : kClMaxRowsG8;
       const bool force16 = h.panel_mode == 3 && cl16_ok<T>();
-      const bool use_clg = ((h.panel_mode == 0 && !use_cl && fm + kClSlack > kClMaxRows) ||
+      const bool use_clg = ((h.panel_mode == 0 && !use_rows) ||
                             force16) &&
                            fm >= h.cl_min_rows && fm + kClSlack <= gmax;
       const bool g16 = use_clg && (force16 || fm + kClSlack > kClMaxRowsG8);
@@ -2960,7 +3060,7 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
           h.cl_scratch_bytes = need;
         }
       }
-      const bool use_sw = !use_cl && !use_clg && fm <= (long long)kSwThreads * kSwRows;
+      const bool use_sw = !use_cl && !use_clg && !use_rows && fm <= (long long)kSwThreads * kSwRows;
       const int sw_smem = kSwSmemBytes;
       // panels a front of big_max_fs candidates needs without delays: each
       // takes nbe - 1 pivots, nbe growing as the remaining rows shrink
@@ -2984,7 +3084,11 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
         budget += panels;
         for (int it = 0; it < panels; it++) {
           if (trace) cudaEventRecord(te[0], s);
-          if (use_cl) {
+          if (use_rows) {
+            const int rc = launch_panel_rows<T>(h.device, B, s, d, nodes, h.ustab, h.pivot_tol,
+                                                row_rows);
+            if (rc) return rc;
+          } else if (use_cl) {
             const int rc = launch_panel_cl<T>(B, cl_smem, s, d, nodes, h.ustab,
                                               h.pivot_tol, cl_rule, (int)fm + kClSlack,
                                               dbg_l);
@@ -3128,6 +3232,10 @@ int factor_numeric(LdlHandle& h, const double* d_vals, cudaStream_t s) {
     }
     if (status & tc::kStatusTimeout) {
       std::fprintf(stderr, "amigo_b200: tensor-core update wait ran out\n");
+      return AB_ERR_CUDA;
+    }
+    if (status & ST_WAIT) {
+      std::fprintf(stderr, "amigo_b200: a cluster panel's wait ran out\n");
       return AB_ERR_CUDA;
     }
     if (status & (ST_POOL_F | ST_POOL_I)) {

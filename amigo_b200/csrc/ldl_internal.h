@@ -38,6 +38,7 @@ enum : int {
   ST_POOL_F = 1,     // FP64 front pool exhausted
   ST_POOL_I = 2,     // int pool exhausted
   ST_NAN = 4,        // non-finite pivot met
+  ST_WAIT = 16,      // a cluster panel's bounded wait ran out
 };
 
 struct DevicePlan {
@@ -119,11 +120,15 @@ struct LdlHandle {
   // f * npiv from which a front is solved by a cluster of CTAs, and from
   // which by the cooperative grid
   long long cluster_entries = 1 << 14;
-  // large-front panels: 0 cluster panels for levels whose largest front has
-  // at least cl_min_rows rows, 1 one-CTA panels only, 2 cluster panels
-  // with the one-CTA panel's widths
+  // large-front panels: 0 one row a thread on clusters sized to the front
+  // (k_big_panel_rows) for levels whose largest front has at least
+  // cl_min_rows rows, one-CTA panels below (default: none, it is the faster
+  // one from the smallest large front on: 32x16 KKT 2.97 ms against 3.31 with
+  // one-CTA panels up to 256 rows and 4.57 up to 768), 1 one-CTA panels only,
+  // 2 cluster panels with the one-CTA panel's widths, 3 the global-scratch
+  // form on clusters of 16
   int panel_mode = 0;
-  int cl_min_rows = 768;
+  int cl_min_rows = 1;
   // global scratch of the cluster panel for fronts past shared memory
   void* cl_scratch = nullptr;
   size_t cl_scratch_bytes = 0;

@@ -136,11 +136,12 @@ int ab_ldl_set_wide_threshold(ab_ldl_t h, long long entries);
 int ab_ldl_set_cluster_threshold(ab_ldl_t h, long long entries);
 
 /* Large-front panel knob.  mode 0 (default): levels whose largest front
- * has at least min_rows rows (default 768) factor their panels on one
- * thread-block cluster of 8 CTAs per front, NB = 32 columns a panel;
- * fronts past what shared memory holds (> 3,008 rows) keep W and L in a
- * global scratch region, on clusters of 8 CTAs to 16,320 rows and of 16
- * (where the device schedules them) to 32,704;
+ * has at least min_rows rows (default 1) factor their panels with one row a
+ * thread on one thread-block cluster per front, of 1 to 16 CTAs by its rows
+ * (to 8,192 rows; 2,048 where the device schedules no clusters of 16), NB =
+ * 32 columns a panel; fronts past that keep W and L in a global scratch
+ * region, on clusters of 8 CTAs to 16,320 rows and of 16 to 32,704; levels
+ * below min_rows take one CTA per front;
  * mode 1: one CTA per front for every level; mode 2: cluster panels with
  * the one-CTA panel's widths, whose results are the one-CTA panel's bit
  * for bit (a test mode); mode 3: the global-scratch form on clusters of 16
