@@ -152,18 +152,19 @@ struct LdlHandle {
   // backward queue and its dependencies (parent in the queue, or -1), done
   // flags per node with an epoch per sweep, the queue counters and the
   // wait-ran-out word
-  // bit 0: work-queue sweeps (default on); bit 1: fronts of at most 128
-  // rows on 128-thread CTAs (off: measured slower)
+  // bit 0: work-queue sweeps (default on); bit 1: in the launches per level,
+  // fronts of at most 128 rows on 128-thread CTAs of their own (off: measured
+  // slower; a queue of such fronts only always runs on 128 threads)
   int solve_queue = 1;
-  int sv_qlevels = 0, sv_qcount = 0, sv_qsmem = 0, sv_qgrid = 0, sv_qsmall_smem = 0;
+  int sv_qlevels = 0, sv_qcount = 0, sv_qsmem = 0, sv_qgrid = 0, sv_precision = 0;
   bool sv_qsmall = false, sv_qgrid_small = false;
   std::vector<int> sv_small_cnt;   // per level: narrow fronts of <= 128 rows
-  std::vector<int> sv_small_smem;  // per level: their front vector bytes
+  std::vector<int> sv_small_smem;  // per level: their shared memory
   std::vector<int> sv_bq_host, sv_dep_host;
   int* sv_bq = nullptr;
   int* sv_dep = nullptr;
-  unsigned* sv_done = nullptr;   // 2 x nn: forward, backward
-  unsigned* sv_ctr = nullptr;    // 4: forward and backward counters, epoch, pad
+  unsigned* sv_done = nullptr;   // forward, backward; per right-hand-side slice, node
+  unsigned* sv_ctr = nullptr;    // forward, backward counters per slice; epoch
   int* sv_err = nullptr;
 };
 

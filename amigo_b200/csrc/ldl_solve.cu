@@ -28,6 +28,12 @@ namespace {
 
 constexpr int NT = kThreads;
 constexpr int SB = 32;  // column block of the triangular solves
+// Right-hand sides solved at the same time: slice y of a launch (blockIdx.y)
+// takes right-hand sides y, y + slices, ...; a front's chain of dependent steps
+// leaves most of the GPU idle, so the slices cost little more than one: eight
+// right-hand sides of the 3D 12x6x6 KKT 10.9 ms one after another, 1.27 ms so
+// (one alone 1.34 with FP32 fronts).
+constexpr int kRhsSlices = 8;
 
 __device__ __forceinline__ int decode_var(int v) { return v >= 0 ? v : -v - 1; }
 
@@ -259,7 +265,7 @@ __device__ void forward_front(const DevicePlan& d, int node, double* x, int nrhs
   double* sL = sm.L;
   int* sK = sm.K;
 
-  for (int rhs = 0; rhs < nrhs; rhs++) {
+  for (int rhs = blockIdx.y; rhs < nrhs; rhs += gridDim.y) {
     // The front vector is worked on in shared memory when it fits (every
     // step of the in-block triangular solve depends on the previous one);
     // its tail is stored in ubuf for the parent.
@@ -311,6 +317,8 @@ __device__ void forward_front(const DevicePlan& d, int node, double* x, int nrhs
   }
 }
 
+#include "solve_front.cuh"
+
 template <class T, int NTH = NT>
 __global__ void __launch_bounds__(NTH)
 k_solve_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
@@ -319,7 +327,12 @@ k_solve_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
   pdl_enter();
   extern __shared__ double sV[];
   __shared__ NarrowSmem sm;
-  forward_front<T, NTH>(d, nodes[blockIdx.x], x, nrhs, ldx, ubuf, uoff, smem_doubles, sV, sm);
+  const int node = nodes[blockIdx.x];
+  if (staged_bytes<T>(d.f[node], d.npiv[node]) <= 8 * (size_t)smem_doubles)
+    forward_staged<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, reinterpret_cast<char*>(sV),
+                           []() {});
+  else
+    forward_front<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, smem_doubles, sV, sm);
 }
 
 // Backward solve of one front by the whole CTA.
@@ -335,7 +348,7 @@ __device__ void backward_front(const DevicePlan& d, int node, double* x, int nrh
   const T* L = reinterpret_cast<const T*>(d.fpool) + d.foff[node];
   double* sL = sm.L;
   int* sK = sm.K;
-  for (int rhs = 0; rhs < nrhs; rhs++) {
+  for (int rhs = blockIdx.y; rhs < nrhs; rhs += gridDim.y) {
     double* V = f <= smem_doubles ? sV : ubuf + uoff[node] + (long long)rhs * f;
     double* xr = x + (long long)rhs * ldx;
     // pivots: their forward values (written to x by the forward sweep);
@@ -381,7 +394,11 @@ k_solve_backward(DevicePlan d, const int* __restrict__ nodes, double* x,
   pdl_enter();
   extern __shared__ double sV[];
   __shared__ NarrowSmem sm;
-  backward_front<T, NTH>(d, nodes[blockIdx.x], x, nrhs, ldx, ubuf, uoff, smem_doubles, sV, sm);
+  const int node = nodes[blockIdx.x];
+  if (staged_bytes<T>(d.f[node], d.npiv[node]) <= 8 * (size_t)smem_doubles)
+    backward_staged<T, NTH>(d, node, x, nrhs, ldx, reinterpret_cast<char*>(sV), []() {});
+  else
+    backward_front<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, smem_doubles, sV, sm);
 }
 
 // Narrow fronts of at most kSmallRows rows run on CTAs of kSmallThreads
@@ -389,6 +406,7 @@ k_solve_backward(DevicePlan d, const int* __restrict__ nodes, double* x,
 // so the same bits).
 constexpr int kSmallRows = 128;
 constexpr int kSmallThreads = 128;
+constexpr int kSolveSms = 148;  // CTAs of a launch that run at once, one per SM
 
 // ---------------------------------------------------------------------------
 // Work-queue sweeps over the levels whose fronts are all narrow: one launch
@@ -416,7 +434,7 @@ __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
 __device__ __forceinline__ void wait_done(const unsigned* flag, unsigned epoch, int* err) {
   for (long long it = 0; it < kQueuePolls; it++) {
     if (ld_acquire(flag) == epoch) return;
-    __nanosleep(64);
+    if (it >= 16) __nanosleep(64);
   }
   atomicOr(err, 1);
 }
@@ -437,15 +455,13 @@ __device__ __forceinline__ void mark_done(unsigned* flag, unsigned epoch) {
   if (threadIdx.x == 0) st_release(flag, epoch);
 }
 
-// Start of a solve's two queued sweeps: zero both queue counters and move
-// to the next epoch (ctr[2]).  The epoch lives in device memory, so a
+// Start of a solve's two queued sweeps: zero the queue counters (forward and
+// backward of every right-hand-side slice) and move to the next epoch.  The epoch lives in device memory, so a
 // captured CUDA graph of a solve takes a new epoch on every replay.
+constexpr int kEpochWord = 2 * kRhsSlices;
 __global__ void k_sweep_begin(unsigned* ctr) {
-  if (threadIdx.x == 0) {
-    ctr[0] = 0u;
-    ctr[1] = 0u;
-    ctr[2] = ctr[2] + 1u;
-  }
+  if (threadIdx.x < 2 * kRhsSlices) ctr[threadIdx.x] = 0u;
+  if (threadIdx.x == 0) ctr[kEpochWord] = ctr[kEpochWord] + 1u;
 }
 
 template <class T, int NTH = NT>
@@ -458,15 +474,25 @@ k_solve_forward_q(DevicePlan d, const int* __restrict__ nodes, int count, double
   extern __shared__ double sV[];
   __shared__ NarrowSmem sm;
   __shared__ int s_idx;
+  ctr += blockIdx.y;
+  done += (size_t)blockIdx.y * d.nn;
   const unsigned epoch = *ep;
   for (;;) {
     const int idx = queue_next(ctr, count, &s_idx);
     if (idx < 0) break;
     const int node = nodes[idx];
-    for (int q = d.kid_ptr[node] + threadIdx.x; q < d.kid_ptr[node + 1]; q += NTH)
-      wait_done(done + d.kids[q], epoch, err);
-    __syncthreads();
-    forward_front<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, smem_doubles, sV, sm);
+    auto wait = [&]() {
+      for (int q = d.kid_ptr[node] + threadIdx.x; q < d.kid_ptr[node + 1]; q += NTH)
+        wait_done(done + d.kids[q], epoch, err);
+    };
+    if (staged_bytes<T>(d.f[node], d.npiv[node]) <= 8 * (size_t)smem_doubles) {
+      forward_staged<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, reinterpret_cast<char*>(sV),
+                             wait);
+    } else {
+      wait();
+      __syncthreads();
+      forward_front<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, smem_doubles, sV, sm);
+    }
     mark_done(done + node, epoch);
   }
 }
@@ -481,14 +507,23 @@ k_solve_backward_q(DevicePlan d, const int* __restrict__ nodes,
   extern __shared__ double sV[];
   __shared__ NarrowSmem sm;
   __shared__ int s_idx;
+  ctr += blockIdx.y;
+  done += (size_t)blockIdx.y * d.nn;
   const unsigned epoch = *ep;
   for (;;) {
     const int idx = queue_next(ctr, count, &s_idx);
     if (idx < 0) break;
     const int node = nodes[idx];
-    if (threadIdx.x == 0 && dep[idx] >= 0) wait_done(done + dep[idx], epoch, err);
-    __syncthreads();
-    backward_front<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, smem_doubles, sV, sm);
+    auto wait = [&]() {
+      if (threadIdx.x == 0 && dep[idx] >= 0) wait_done(done + dep[idx], epoch, err);
+    };
+    if (staged_bytes<T>(d.f[node], d.npiv[node]) <= 8 * (size_t)smem_doubles) {
+      backward_staged<T, NTH>(d, node, x, nrhs, ldx, reinterpret_cast<char*>(sV), wait);
+    } else {
+      wait();
+      __syncthreads();
+      backward_front<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, smem_doubles, sV, sm);
+    }
     mark_done(done + node, epoch);
   }
 }
@@ -510,6 +545,48 @@ __device__ __forceinline__ void copy_cg(double* dst, const double* src, int n) {
   for (int t = threadIdx.x; t < n; t += NT) dst[t] = __ldcg(src + t);
 }
 
+// Shared memory of a cluster front: its vector (CTA 0; the other CTAs hold the
+// pivots' values there), the children's row positions, the pivot kinds, two diagonal blocks and the partial sums of the
+// contribution rows.
+constexpr int DB = (SB + 1) * (SB + 1);
+struct CluSmem {
+  double* V;
+  double* part;   // NT
+  double* diag;   // 2 x DB
+  int* P;         // clu_positions(f)
+  unsigned char* K;
+};
+// Row positions held (past 8,192 rows the vector takes their room).
+__host__ __device__ __forceinline__ int clu_positions(int f) { return f <= 8192 ? 2 * f : 0; }
+__host__ __device__ __forceinline__ size_t clu_bytes(int f, int npiv) {
+  return ((size_t)f + NT + 2 * DB) * 8 + (size_t)clu_positions(f) * 4 + npiv + 16;
+}
+__device__ __forceinline__ CluSmem clu_smem(double* raw, int f) {
+  CluSmem m;
+  m.V = raw;
+  m.part = raw + f;
+  m.diag = m.part + NT;
+  m.P = reinterpret_cast<int*>(m.diag + 2 * DB);
+  m.K = reinterpret_cast<unsigned char*>(m.P + clu_positions(f));
+  return m;
+}
+// The diagonal block of columns [jb, je) into `dst` (in flight until cp_wait);
+// T entries, leading dimension SB + 1.
+template <class T>
+__device__ __forceinline__ void fetch_diag(const T* L, int f, int jb, int bw, double* dst) {
+  T* o = reinterpret_cast<T*>(dst);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int j = warp; j < bw; j += NT / 32)
+    for (int i = lane; i < bw; i += 32)
+      if (i >= j) cp_async_el(o + i + j * (SB + 1), L + jb + i + (size_t)(jb + j) * f);
+}
+
+// CTA 0's part is a chain of 32-column blocks: the block's diagonal is in
+// shared memory and its entries of the next 256 rows in registers before its
+// turn comes (loaded while the previous block is solved and applied), so a
+// block costs the warp's triangular solve and 32 multiply-adds a row, without
+// a global load in between.  One solve of the 2D SIMP 128x64 KKT (fronts of
+// ~1,100 rows and ~280 pivots, one after another) 3.77 -> 2.44 ms.
 template <class T>
 __global__ void __launch_bounds__(NT, 1)
 k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
@@ -518,9 +595,6 @@ k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double sm[];
-  __shared__ double sL[(SB + 1) * (SB + 1)];
-  __shared__ int sK[SB + 1];
-  __shared__ int s_choff;
   const int cr = (int)cluster.block_rank();
   const int node = nodes[blockIdx.x / CS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -529,41 +603,99 @@ k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
   const int* fvars = d.ipool + d.ioff[node];
   const int* kind = fvars + 3 * f;
   const T* L = reinterpret_cast<const T*>(d.fpool) + d.foff[node];
-  double* sv = sm;                 // CTA 0: pivot values; others: y1 copy
-  double* part = sm + npiv;        // NWARP x 32 partial sums
-  for (int rhs = 0; rhs < nrhs; rhs++) {
+  const CluSmem m = clu_smem(sm, f);
+  double* V = m.V;
+  const int ns = d.ns[node], ndin = d.ndin[node], fs = ns + ndin;
+  const int* fsinv = fvars + 2 * f;
+  const int q0 = d.kid_ptr[node], q1 = d.kid_ptr[node + 1];
+  auto position = [&](int c, int ndc, int choff, int a) {
+    int pos;
+    if (a < ndc) {
+      pos = choff + a;
+    } else {
+      const int r0 = d.cmap[d.cptr[c] + a - ndc];
+      pos = r0 < ns ? r0 : r0 + ndin;
+    }
+    return pos < fs ? fsinv[pos] : pos;
+  };
+  int held = 0;
+  if (cr == 0) {
+    for (int j = tid; j < npiv; j += NT) m.K[j] = (unsigned char)kind[j];
+    for (int q = q0, choff = ns, at = 0; q < q1; q++) {
+      const int c = d.kids[q], ndc = d.ndel[c], cc = d.f[c] - d.npiv[c];
+      if (at + cc > clu_positions(f)) break;
+      for (int a = tid; a < cc; a += NT) m.P[at + a] = position(c, ndc, choff, a);
+      at += cc;
+      choff += ndc;
+      held = q + 1 - q0;
+    }
+  }
+  for (int rhs = blockIdx.y; rhs < nrhs; rhs += gridDim.y) {
     double* G = ubuf + uoff[node] + (long long)rhs * f;
     double* xr = x + (long long)rhs * ldx;
     if (cr == 0) {
-      assemble_front_vector(d, node, G, xr, ubuf, uoff, rhs, &s_choff);
+      for (int r = tid; r < f; r += NT) V[r] = 0.0;
       __syncthreads();
-      for (int t = tid; t < npiv; t += NT) sv[t] = G[t];
+      const int vb = d.var_ptr[node];
+      for (int r = tid; r < ns; r += NT) V[fsinv[r]] = xr[d.vars[vb + r]];
       __syncthreads();
-      for (int jb = 0; jb < npiv;) {
-        const int je = block_end(kind, jb, npiv);
-        const int bw = je - jb;
-        for (int t = tid; t < bw * bw; t += NT) {
-          const int i = t % bw, j = t / bw;
-          sL[i + j * (SB + 1)] = L[jb + i + (size_t)(jb + j) * f];
-        }
-        for (int t = tid; t < bw; t += NT) sK[t] = kind[jb + t];
+      auto end_of = [&](int jb) {
+        int je = min(jb + SB, npiv);
+        if (je < npiv && m.K[je - 1] == 1) je++;
+        return je;
+      };
+      int jb = 0, je = npiv > 0 ? end_of(0) : 0, buf = 0;
+      fetch_diag<T>(L, f, 0, je, m.diag);
+      for (int q = q0, choff = ns, at = 0; q < q1; q++) {
+        const int c = d.kids[q], ndc = d.ndel[c], npc = d.npiv[c], cc = d.f[c] - npc;
+        const double* uc = ubuf + uoff[c] + (long long)rhs * d.f[c] + npc;
+        const bool in_p = q - q0 < held;
+        for (int a = tid; a < cc; a += NT)
+          V[in_p ? m.P[at + a] : position(c, ndc, choff, a)] += __ldcg(uc + a);
         __syncthreads();
-        if (warp == 0) warp_lower_solve<2>(sL, SB + 1, sK, bw, sv + jb, lane);
-        __syncthreads();
-        // the pivot rows below the block
-        for (int i = je + tid; i < npiv; i += NT)
-          sv[i] -= dot_strided(L + i + (size_t)jb * f, (size_t)f, bw,
-                               [&](int j) { return sv[jb + j]; });
-        __syncthreads();
-        jb = je;
+        at += cc;
+        choff += ndc;
       }
-      for (int t = tid; t < npiv; t += NT) G[t] = sv[t];
+      while (jb < npiv) {
+        const int bw = je - jb;
+        // the block's entries of this thread's row, its 33rd column apart
+        const int i0 = je + tid;
+        const T* Li = L + (i0 < npiv ? i0 : 0) + (size_t)jb * f;
+        T a[SB];
+#pragma unroll
+        for (int j = 0; j < SB; j++) a[j] = i0 < npiv && j < bw ? Li[(size_t)j * f] : T(0);
+        const T a32 = i0 < npiv && bw > SB ? Li[(size_t)SB * f] : T(0);
+        cp_wait();
+        __syncthreads();  // the diagonal block; the rows' updates of the last one
+        if (warp == 0)
+          lower_block<T>(reinterpret_cast<const T*>(m.diag + buf * DB), SB + 1, m.K + jb, bw,
+                         V + jb, lane);
+        const int jn = je < npiv ? end_of(je) : je;
+        if (je < npiv) fetch_diag<T>(L, f, je, jn - je, m.diag + (buf ^ 1) * DB);
+        __syncthreads();
+        if (i0 < npiv) {
+          double acc = 0.0;
+#pragma unroll
+          for (int j = 0; j < SB; j++)
+            if (j < bw) acc = __fma_rn((double)a[j], V[jb + j], acc);
+          if (bw > SB) acc = __fma_rn((double)a32, V[jb + SB], acc);
+          V[i0] -= acc;
+        }
+        for (int i = i0 + NT; i < npiv; i += NT)
+          V[i] -= dot_strided(L + i + (size_t)jb * f, (size_t)f, bw,
+                              [&](int j) { return V[jb + j]; });
+        jb = je;
+        je = jn;
+        buf ^= 1;
+      }
+      __syncthreads();
+      for (int t = tid; t < f; t += NT) G[t] = V[t];
     }
     cluster.sync();
     // contribution rows: G[i] -= L21[i, :] y1, 32-row strips over the
     // cluster's CTAs, the pivot columns split over the CTA's warps and the
     // warps' partial sums added in a fixed order
-    if (cr != 0) copy_cg(sv, G, npiv);
+    if (cr != 0) copy_cg(V, G, npiv);
     __syncthreads();
     const int ncr = f - npiv;
     const int nstrip = (ncr + 31) / 32;
@@ -574,12 +706,12 @@ k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
       double acc = 0.0;
       if (i < f && j1 > j0)
         acc = dot_strided(L + i + (size_t)j0 * f, (size_t)f, j1 - j0,
-                          [&](int j) { return sv[j0 + j]; });
-      part[warp * 32 + lane] = acc;
+                          [&](int j) { return V[j0 + j]; });
+      m.part[warp * 32 + lane] = acc;
       __syncthreads();
       if (warp == 0 && i < f) {
         double s = 0.0;
-        for (int w = 0; w < NWARP; w++) s += part[w * 32 + lane];
+        for (int w = 0; w < NWARP; w++) s += m.part[w * 32 + lane];
         G[i] = __ldcg(G + i) - s;
       }
       __syncthreads();
@@ -587,22 +719,16 @@ k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
     // D^{-1} and the pivots' values (CTA 0, from its shared copy)
     if (cr == 0) {
       for (int j = tid; j < npiv; j += NT) {
-        const int kd = kind[j];
-        double v = sv[j];
+        const int kd = m.K[j];
+        double v;
         if (kd == 0) {
-          v = sv[j] / (double)L[j + (size_t)j * f];
-        } else if (kd == 1) {
-          const double d11 = L[j + (size_t)j * f];
-          const double d21 = L[j + 1 + (size_t)j * f];
-          const double d22 = L[j + 1 + (size_t)(j + 1) * f];
-          const double inv = inv2x2(d11, d21, d22);
-          v = piv2_first(inv, d21, d22, sv[j], sv[j + 1]);
+          v = V[j] / (double)L[j + (size_t)j * f];
         } else {
-          const double d11 = L[j - 1 + (size_t)(j - 1) * f];
-          const double d21 = L[j + (size_t)(j - 1) * f];
-          const double d22 = L[j + (size_t)j * f];
+          const T* Lf = L + (j - kd + 1) * ((size_t)f + 1);  // the pair's first diagonal
+          const double d11 = Lf[0], d21 = Lf[1], d22 = Lf[f + 1];
           const double inv = inv2x2(d11, d21, d22);
-          v = piv2_second(inv, d11, d21, sv[j - 1], sv[j]);
+          v = kd == 1 ? piv2_first(inv, d21, d22, V[j], V[j + 1])
+                      : piv2_second(inv, d11, d21, V[j - 1], V[j]);
         }
         xr[decode_var(fvars[j])] = v;
       }
@@ -619,8 +745,6 @@ k_clu_backward(DevicePlan d, const int* __restrict__ nodes, double* x,
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double sm[];
-  __shared__ double sL[(SB + 1) * (SB + 1)];
-  __shared__ int sK[SB + 1];
   const int cr = (int)cluster.block_rank();
   const int node = nodes[blockIdx.x / CS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -630,9 +754,12 @@ k_clu_backward(DevicePlan d, const int* __restrict__ nodes, double* x,
   const int* kind = fvars + 3 * f;
   const T* L = reinterpret_cast<const T*>(d.fpool) + d.foff[node];
   const int ncr = f - npiv;
-  double* sx = sm;            // contribution rows' final values
-  double* sv = sm + ncr;      // CTA 0: pivot values
-  for (int rhs = 0; rhs < nrhs; rhs++) {
+  const CluSmem m = clu_smem(sm, f);
+  double* sx = m.V + npiv;    // contribution rows' final values
+  double* V = m.V;            // CTA 0: pivot values
+  if (cr == 0)
+    for (int j = tid; j < npiv; j += NT) m.K[j] = (unsigned char)kind[j];
+  for (int rhs = blockIdx.y; rhs < nrhs; rhs += gridDim.y) {
     double* G = ubuf + uoff[node] + (long long)rhs * f;
     double* xr = x + (long long)rhs * ldx;
     for (int r = tid; r < ncr; r += NT) sx[r] = xr[fvars[npiv + r]];
@@ -646,30 +773,57 @@ k_clu_backward(DevicePlan d, const int* __restrict__ nodes, double* x,
     }
     cluster.sync();
     if (cr == 0) {
-      for (int t = tid; t < npiv; t += NT) sv[t] = __ldcg(G + t);
-      __syncthreads();
-      int je = npiv;
+      for (int t = tid; t < npiv; t += NT) V[t] = __ldcg(G + t);
+      auto begin_of = [&](int je) {
+        int jb = max(je - SB, 0);
+        if (jb > 0 && m.K[jb] == 2) jb--;  // keep 2x2 pairs together
+        return jb;
+      };
+      int je = npiv, jb = npiv > 0 ? begin_of(npiv) : 0, buf = 0;
+      if (npiv > 0) fetch_diag<T>(L, f, jb, je - jb, m.diag);
       while (je > 0) {
-        int jb = je - SB > 0 ? je - SB : 0;
-        if (jb > 0 && kind[jb] == 2) jb--;  // keep 2x2 pairs together
-        // t[j] -= sum_{je <= i < npiv} L[i, j] t[i] for j in [jb, je)
-        for (int j = jb + warp; j < je; j += NWARP) {
-          const double acc = warp_sum_down(lane_dot(L + (size_t)j * f, je, npiv, lane,
-                                                    [&](int i) { return sv[i]; }));
-          if (lane == 0) sv[j] -= acc;
+        // t[j] -= sum_{je <= i < npiv} L[i, j] t[i] for j in [jb, je): four or
+        // five columns a warp together, the entries of the rows that do not
+        // wait for the last block loaded before it was done
+        constexpr int CW = (SB + 1 + NWARP - 1) / NWARP, RW = 8;
+        const int jw = jb + warp;  // this warp's columns: jw, jw + NWARP, ...
+        T pre[CW][RW];
+#pragma unroll
+        for (int u = 0; u < CW; u++)
+#pragma unroll
+          for (int r = 0; r < RW; r++) {
+            const int j = jw + NWARP * u, i = je + lane + 32 * r;
+            pre[u][r] = j < je && i < npiv ? L[i + (size_t)j * f] : T(0);
+          }
+        __syncthreads();  // the last block's values
+#pragma unroll
+        for (int u = 0; u < CW; u++) {
+          const int j = jw + NWARP * u;
+          if (j >= je) break;
+          double acc = 0.0;
+#pragma unroll
+          for (int r = 0; r < RW; r++) {
+            const int i = je + lane + 32 * r;
+            if (i < npiv) acc = __fma_rn((double)pre[u][r], V[i], acc);
+          }
+          for (int i = je + lane + 32 * RW; i < npiv; i += 32)
+            acc = __fma_rn((double)L[i + (size_t)j * f], V[i], acc);
+          acc = warp_sum_down(acc);
+          if (lane == 0) V[j] -= acc;
         }
-        const int bw = je - jb;
-        for (int t = tid; t < bw * bw; t += NT) {
-          const int i = t % bw, j = t / bw;
-          sL[i + j * (SB + 1)] = L[jb + i + (size_t)(jb + j) * f];
-        }
-        for (int t = tid; t < bw; t += NT) sK[t] = kind[jb + t];
+        cp_wait();
         __syncthreads();
-        if (warp == 0) warp_upper_solve<2>(sL, SB + 1, sK, bw, sv + jb, lane);
-        __syncthreads();
+        if (warp == 0)
+          upper_block<T>(reinterpret_cast<const T*>(m.diag + buf * DB), SB + 1, m.K + jb,
+                         je - jb, V + jb, lane);
+        const int jn = jb > 0 ? begin_of(jb) : 0;
+        if (jb > 0) fetch_diag<T>(L, f, jn, jb - jn, m.diag + (buf ^ 1) * DB);
         je = jb;
+        jb = jn;
+        buf ^= 1;
       }
-      for (int j = tid; j < npiv; j += NT) xr[decode_var(fvars[j])] = sv[j];
+      __syncthreads();
+      for (int j = tid; j < npiv; j += NT) xr[decode_var(fvars[j])] = V[j];
     }
     cluster.sync();
   }
@@ -983,7 +1137,7 @@ static int launch_cluster(K kernel, int fronts, int smem, cudaStream_t s,
                           const DevicePlan& d, const int* nodes, double* x,
                           int nrhs, int ldx, double* ubuf, const long long* uoff) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(fronts * CS);
+  cfg.gridDim = dim3(fronts * CS, std::max(1, std::min(nrhs, kRhsSlices)));
   cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = s;
@@ -1007,7 +1161,7 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
   const int L = h.d.num_levels, nn = h.d.nn;
   // unchanged front sizes (the usual case between IPM iterations): keep it
   if (h.sv_f == h.h_f && h.sv_npiv == h.h_npiv && !h.sv_narrow_ptr.empty() &&
-      h.sv_wide_entries == h.wide_entries) {
+      h.sv_wide_entries == h.wide_entries && h.sv_precision == h.factor_precision) {
     h.solve_epoch = h.factor_epoch;
     return 0;
   }
@@ -1026,41 +1180,67 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
   auto cls = [&](int k) {
     const long long e = (long long)h.h_f[k] * h.h_npiv[k];
     if (e >= h.wide_entries) return 2;
-    if (e >= h.cluster_entries && ((long long)h.h_f[k] + NT) * 8 <= kMaxDynSmem) return 1;
+    if (e >= h.cluster_entries) {
+      if ((long long)clu_bytes(h.h_f[k], h.h_npiv[k]) <= kMaxDynSmem) return 1;
+      // (a vector past a CTA's shared memory: the grid, unless it was asked
+      // not to)
+      if (h.wide_entries < (1ll << 40)) return 2;
+    }
     return 0;
   };
   h.sv_small_cnt.assign(L, 0);
   h.sv_small_smem.assign(L, 0);
+  // Shared memory of a launch over `fronts` narrow fronts (size f, pivots p):
+  // their vectors, and the pivot columns of those that fit the cap (the others
+  // read the factor from global memory).  The cap leaves room for as many CTAs
+  // per SM as the launch has fronts for, at most four: with more fronts than
+  // that a front's latency is hidden by the others'.
+  auto stage_cap = [&](int fronts) -> long long {
+    return fronts > 3 * kSolveSms ? 48 * 1024
+                                  : fronts > kSolveSms ? 96 * 1024 : kMaxDynSmem;
+  };
+  auto stage_bytes = [&](int k) -> long long {
+    return (long long)(h.factor_precision == 32
+                           ? staged_bytes<float>(h.h_f[k], h.h_npiv[k])
+                           : staged_bytes<double>(h.h_f[k], h.h_npiv[k]));
+  };
+  auto narrow_smem = [&](const int* list, int count, long long cap) -> int {
+    long long sm = 0;
+    for (int i = 0; i < count; i++) {
+      const long long b = stage_bytes(list[i]);
+      sm = std::max(sm, b <= cap ? b : std::min<long long>(8ll * h.h_f[list[i]], kMaxDynSmem));
+    }
+    return (int)((sm + 15) & ~15ll);
+  };
   for (int l = 0; l < L; l++) {
     h.sv_narrow_ptr[l] = (int)nodes.size();
-    int fm = 0, fsm = 0;
     // narrow fronts: the small ones (kSmallThreads-thread CTAs) first
     for (int pass = 0; pass < 2; pass++)
       for (int q = h.level_ptr[l]; q < h.level_ptr[l + 1]; q++) {
         const int k = h.level_nodes[q];
         if (cls(k) == 0 && (h.h_f[k] <= kSmallRows) == (pass == 0)) {
           nodes.push_back(k);
-          if (pass == 0) {
-            h.sv_small_cnt[l]++;
-            fsm = std::max(fsm, h.h_f[k]);
-          } else {
-            fm = std::max(fm, h.h_f[k]);
-          }
+          if (pass == 0) h.sv_small_cnt[l]++;
         }
       }
-    h.sv_small_smem[l] = fsm * 8;
-    h.sv_narrow_smem[l] =
-        (int)std::min<long long>((long long)fm * 8, kMaxDynSmem);
+    {
+      const int* list = nodes.data() + h.sv_narrow_ptr[l];
+      const int cnt = (int)nodes.size() - h.sv_narrow_ptr[l];
+      const long long cap = stage_cap(cnt);
+      h.sv_small_smem[l] = narrow_smem(list, h.sv_small_cnt[l], cap);
+      // (the launch covers the small fronts too unless they have their own)
+      h.sv_narrow_smem[l] = narrow_smem(list, cnt, cap);
+    }
     h.sv_clu_ptr[l] = (int)nodes.size();
-    int cm = 0;
+    long long cm = 0;
     for (int q = h.level_ptr[l]; q < h.level_ptr[l + 1]; q++) {
       const int k = h.level_nodes[q];
       if (cls(k) == 1) {
         nodes.push_back(k);
-        cm = std::max(cm, h.h_f[k]);
+        cm = std::max(cm, (long long)clu_bytes(h.h_f[k], h.h_npiv[k]));
       }
     }
-    h.sv_clu_smem[l] = (int)std::min<long long>(((long long)cm + NT) * 8, kMaxDynSmem);
+    h.sv_clu_smem[l] = (int)cm;
     h.sv_wide_ptr[l] = (int)nodes.size();
     for (int q = h.level_ptr[l]; q < h.level_ptr[l + 1]; q++) {
       const int k = h.level_nodes[q];
@@ -1087,12 +1267,8 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
   h.sv_qlevels = ql >= 2 ? ql : 0;
   h.sv_qcount = h.sv_qlevels ? h.sv_narrow_ptr[h.sv_qlevels] : 0;
   h.sv_qsmall = true;
-  int qsm = 0;
-  for (int l = 0; l < h.sv_qlevels; l++) {
+  for (int l = 0; l < h.sv_qlevels; l++)
     if (h.sv_small_cnt[l] != h.sv_clu_ptr[l] - h.sv_narrow_ptr[l]) h.sv_qsmall = false;
-    qsm = std::max(qsm, h.sv_small_smem[l]);
-  }
-  h.sv_qsmall_smem = qsm;
   if (h.sv_qcount) {
     const int qc = h.sv_qcount;
     // position of each queued node in the forward order
@@ -1102,9 +1278,7 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
     std::vector<int>& dep = h.sv_dep_host;
     bq.resize(qc);
     dep.resize(qc);
-    int sm = 0;
-    for (int l = 0; l < h.sv_qlevels; l++) sm = std::max(sm, h.sv_narrow_smem[l]);
-    h.sv_qsmem = sm;
+    h.sv_qsmem = narrow_smem(nodes.data(), qc, stage_cap(qc));
     for (int i = 0; i < qc; i++) {
       const int k = nodes[qc - 1 - i];
       const int par = h.sym.node_parent[k];
@@ -1114,11 +1288,13 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
     if (!h.sv_bq) {
       SCUDA(cudaMalloc((void**)&h.sv_bq, std::max(nn, 1) * sizeof(int)));
       SCUDA(cudaMalloc((void**)&h.sv_dep, std::max(nn, 1) * sizeof(int)));
-      SCUDA(cudaMalloc((void**)&h.sv_done, 2 * (size_t)std::max(nn, 1) * sizeof(unsigned)));
-      SCUDA(cudaMalloc((void**)&h.sv_ctr, 4 * sizeof(unsigned)));
+      SCUDA(cudaMalloc((void**)&h.sv_done,
+                       2 * kRhsSlices * (size_t)std::max(nn, 1) * sizeof(unsigned)));
+      SCUDA(cudaMalloc((void**)&h.sv_ctr, (kEpochWord + 1) * sizeof(unsigned)));
       SCUDA(cudaMalloc((void**)&h.sv_err, sizeof(int)));
-      SCUDA(cudaMemsetAsync(h.sv_done, 0, 2 * (size_t)std::max(nn, 1) * sizeof(unsigned), s));
-      SCUDA(cudaMemsetAsync(h.sv_ctr, 0, 4 * sizeof(unsigned), s));
+      SCUDA(cudaMemsetAsync(h.sv_done, 0,
+                            2 * kRhsSlices * (size_t)std::max(nn, 1) * sizeof(unsigned), s));
+      SCUDA(cudaMemsetAsync(h.sv_ctr, 0, (kEpochWord + 1) * sizeof(unsigned), s));
       SCUDA(cudaMemsetAsync(h.sv_err, 0, sizeof(int), s));
     }
     SCUDA(cudaMemcpyAsync(h.sv_bq, bq.data(), qc * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -1129,6 +1305,7 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
   h.sv_npiv = h.h_npiv;
   h.sv_fwd_grid.clear();
   h.sv_wide_entries = h.wide_entries;
+  h.sv_precision = h.factor_precision;
   h.solve_epoch = h.factor_epoch;
   return 0;
 }
@@ -1145,6 +1322,18 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                kMaxDynSmem));
     SCUDA(cudaFuncSetAttribute(k_solve_backward<T>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kMaxDynSmem));
+    SCUDA(cudaFuncSetAttribute(k_solve_forward<T, kSmallThreads>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kMaxDynSmem));
+    SCUDA(cudaFuncSetAttribute(k_solve_backward<T, kSmallThreads>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kMaxDynSmem));
+    SCUDA(cudaFuncSetAttribute(k_solve_forward_q<T, kSmallThreads>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kMaxDynSmem));
+    SCUDA(cudaFuncSetAttribute(k_solve_backward_q<T, kSmallThreads>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                kMaxDynSmem));
     SCUDA(cudaFuncSetAttribute(k_solve_forward_q<T>,
@@ -1207,10 +1396,12 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
   }
   const bool queue = (h.solve_queue & 1) && h.sv_qcount > 0;
   const bool small = (h.solve_queue & 2) != 0;
-  const bool qsmall = queue && small && h.sv_qsmall;
+  // (a queue of fronts of at most 128 rows only: 128-thread CTAs)
+  const bool qsmall = queue && h.sv_qsmall;
   const int qth = qsmall ? kSmallThreads : NT;
-  const int qsm = qsmall ? h.sv_qsmall_smem : h.sv_qsmem;
-  const unsigned* ep = h.sv_ctr + 2;   // this solve's epoch, set on the device
+  const int qsm = h.sv_qsmem;
+  const unsigned* ep = h.sv_ctr + kEpochWord;   // this solve's epoch, set on the device
+  const int slices = std::max(1, std::min(nrhs, kRhsSlices));
   if (queue) {
     if (h.sv_qgrid == 0 || h.sv_qgrid_small != qsmall) {
       // CTAs resident at once, at most one per queued front
@@ -1229,12 +1420,12 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
     { k_sweep_begin<<<1, 32, 0, s>>>(h.sv_ctr); ab::count_launch(); }
     SCUDA(cudaGetLastError());
     if (qsmall)
-      SCUDA(launch_pdl(k_solve_forward_q<T, kSmallThreads>, dim3(h.sv_qgrid), dim3(qth),
+      SCUDA(launch_pdl(k_solve_forward_q<T, kSmallThreads>, dim3(h.sv_qgrid, slices), dim3(qth),
                        (size_t)qsm, s, d, (const int*)h.sv_nodes, h.sv_qcount, d_x, nrhs,
                        ldx, h.ubuf, (const long long*)h.uoff, qsm / 8, h.sv_ctr, h.sv_done,
                        ep, h.sv_err));
     else
-      SCUDA(launch_pdl(k_solve_forward_q<T>, dim3(h.sv_qgrid), dim3(qth), (size_t)qsm, s, d,
+      SCUDA(launch_pdl(k_solve_forward_q<T>, dim3(h.sv_qgrid, slices), dim3(qth), (size_t)qsm, s, d,
                        (const int*)h.sv_nodes, h.sv_qcount, d_x, nrhs, ldx, h.ubuf,
                        (const long long*)h.uoff, qsm / 8, h.sv_ctr, h.sv_done, ep,
                        h.sv_err));
@@ -1245,7 +1436,7 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
     int b = h.sv_narrow_ptr[l], cnt = h.sv_clu_ptr[l] - b;
     if (small && h.sv_small_cnt[l]) {
       const int sc = h.sv_small_cnt[l];
-      SCUDA(launch_pdl(k_solve_forward<T, kSmallThreads>, dim3(sc), dim3(kSmallThreads),
+      SCUDA(launch_pdl(k_solve_forward<T, kSmallThreads>, dim3(sc, slices), dim3(kSmallThreads),
                        (size_t)h.sv_small_smem[l], s, d, (const int*)(h.sv_nodes + b), d_x,
                        nrhs, ldx, h.ubuf, (const long long*)h.uoff, h.sv_small_smem[l] / 8));
       ab::count_launch();
@@ -1253,7 +1444,7 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
       cnt -= sc;
     }
     if (cnt) {
-      SCUDA(launch_pdl(k_solve_forward<T>, dim3(cnt), dim3(NT), (size_t)h.sv_narrow_smem[l],
+      SCUDA(launch_pdl(k_solve_forward<T>, dim3(cnt, slices), dim3(NT), (size_t)h.sv_narrow_smem[l],
                        s, d, h.sv_nodes + b, d_x, nrhs, ldx, h.ubuf, h.uoff,
                        h.sv_narrow_smem[l] / 8));
       ab::count_launch();
@@ -1284,7 +1475,7 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
     int b = h.sv_narrow_ptr[l], cnt = h.sv_clu_ptr[l] - b;
     if (small && h.sv_small_cnt[l]) {
       const int sc = h.sv_small_cnt[l];
-      SCUDA(launch_pdl(k_solve_backward<T, kSmallThreads>, dim3(sc), dim3(kSmallThreads),
+      SCUDA(launch_pdl(k_solve_backward<T, kSmallThreads>, dim3(sc, slices), dim3(kSmallThreads),
                        (size_t)h.sv_small_smem[l], s, d, (const int*)(h.sv_nodes + b), d_x,
                        nrhs, ldx, h.ubuf, (const long long*)h.uoff, h.sv_small_smem[l] / 8));
       ab::count_launch();
@@ -1292,7 +1483,7 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
       cnt -= sc;
     }
     if (cnt) {
-      SCUDA(launch_pdl(k_solve_backward<T>, dim3(cnt), dim3(NT), (size_t)h.sv_narrow_smem[l],
+      SCUDA(launch_pdl(k_solve_backward<T>, dim3(cnt, slices), dim3(NT), (size_t)h.sv_narrow_smem[l],
                        s, d, h.sv_nodes + b, d_x, nrhs, ldx, h.ubuf, h.uoff,
                        h.sv_narrow_smem[l] / 8));
       ab::count_launch();
@@ -1319,15 +1510,15 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
   }
   if (queue) {
     if (qsmall)
-      SCUDA(launch_pdl(k_solve_backward_q<T, kSmallThreads>, dim3(h.sv_qgrid), dim3(qth),
+      SCUDA(launch_pdl(k_solve_backward_q<T, kSmallThreads>, dim3(h.sv_qgrid, slices), dim3(qth),
                        (size_t)qsm, s, d, (const int*)h.sv_bq, (const int*)h.sv_dep,
                        h.sv_qcount, d_x, nrhs, ldx, h.ubuf, (const long long*)h.uoff,
-                       qsm / 8, h.sv_ctr + 1, h.sv_done + d.nn, ep, h.sv_err));
+                       qsm / 8, h.sv_ctr + kRhsSlices, h.sv_done + (size_t)kRhsSlices * d.nn, ep, h.sv_err));
     else
-      SCUDA(launch_pdl(k_solve_backward_q<T>, dim3(h.sv_qgrid), dim3(qth), (size_t)qsm, s, d,
+      SCUDA(launch_pdl(k_solve_backward_q<T>, dim3(h.sv_qgrid, slices), dim3(qth), (size_t)qsm, s, d,
                        (const int*)h.sv_bq, (const int*)h.sv_dep, h.sv_qcount, d_x, nrhs,
-                       ldx, h.ubuf, (const long long*)h.uoff, qsm / 8, h.sv_ctr + 1,
-                       h.sv_done + d.nn, ep, h.sv_err));
+                       ldx, h.ubuf, (const long long*)h.uoff, qsm / 8, h.sv_ctr + kRhsSlices,
+                       h.sv_done + (size_t)kRhsSlices * d.nn, ep, h.sv_err));
     ab::count_launch();
   }
   if (trace && queue) {
