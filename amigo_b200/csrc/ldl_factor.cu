@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "../../include/amigo_b200.h"
+#include "cluster_msg.cuh"
 #include "ldl_internal.h"
 #include "launch_count.h"
 #include "tc_update.cuh"
@@ -2659,6 +2660,7 @@ k_big_panel_cl(DevicePlan d, const int* __restrict__ nodes, double ustab,
   }
 }
 
+#include "pivot_fold.cuh"
 #include "panel_rows.cuh"
 
 template <class T>

@@ -20,6 +20,7 @@
 #include <cstdlib>
 #include <vector>
 
+#include "cluster_msg.cuh"
 #include "ldl_internal.h"
 #include "launch_count.h"
 
@@ -531,47 +532,57 @@ k_solve_backward_q(DevicePlan d, const int* __restrict__ nodes,
 
 // ---------------------------------------------------------------------------
 // Mid-size fronts: one thread-block cluster of CS CTAs per front.  CTA 0
-// solves the pivot block (the blocked triangular solve of the narrow
-// kernel, over the pivot rows only, with the front vector's pivot part in
-// its shared memory); the contribution rows' product with the pivot block
-// (the update vector passed to the parent, forward; the pivots' right-hand
-// side correction, backward) is spread over all CS CTAs, which read the
-// front's L21 once.  The cluster barrier orders CTA 0's results before the
-// other CTAs read them from HBM (cluster-scope release / acquire).
+// solves the pivot block, a chain of 32-column blocks; the contribution rows'
+// product with it (the update vector passed to the parent, forward; the
+// pivots' right-hand side correction, backward) is spread over the other CTAs,
+// which read the front's L21 once.  The two overlap: forward, a block's values
+// are sent to the other CTAs as soon as they are known; backward, the other
+// CTAs send the columns' corrections, last block first, and CTA 0 takes a block
+// when its columns are there.  Everything that does not depend on another
+// front's values is fetched before the previous launch of the solve is done
+// (the factor was finished before the solve's first launch, see launch_solve).
 constexpr int CS = 8;
 
-// dst[0:n] = src[0:n] from L2 (src may have been written by another CTA).
-__device__ __forceinline__ void copy_cg(double* dst, const double* src, int n) {
-  for (int t = threadIdx.x; t < n; t += NT) dst[t] = __ldcg(src + t);
-}
+constexpr int CW = CS - 1;                // CTAs that take the contribution rows
+constexpr int DB = (SB + 1) * (SB + 1);   // a diagonal block
+constexpr int kCluKids = 8;               // children whose sizes are held
+constexpr int kCluWait = 2;               // error word bit: a message's wait ran out
 
-// Shared memory of a cluster front: its vector (CTA 0; the other CTAs hold the
-// pivots' values there), the children's row positions, the pivot kinds, two diagonal blocks and the partial sums of the
-// contribution rows.
-constexpr int DB = (SB + 1) * (SB + 1);
+// Shared memory of a cluster front: its vector (CTA 0; backward the pivots'
+// values and their corrections) or the pivots' values and sums of rows past 256
+// (the other CTAs; backward the contribution rows' values), two diagonal blocks, an mbarrier per block, the children's row
+// positions, the blocks' first columns and the pivot kinds.
 struct CluSmem {
   double* V;
-  double* part;   // NT
-  double* diag;   // 2 x DB
-  int* P;         // clu_positions(f)
+  double* diag;              // 2 x DB
+  unsigned long long* bar;   // a block each
+  int* P;                    // clu_positions(f)
+  unsigned short* jb;        // blocks + 1
   unsigned char* K;
 };
 // Row positions held (past 8,192 rows the vector takes their room).
 __host__ __device__ __forceinline__ int clu_positions(int f) { return f <= 8192 ? 2 * f : 0; }
-__host__ __device__ __forceinline__ size_t clu_bytes(int f, int npiv) {
-  return ((size_t)f + NT + 2 * DB) * 8 + (size_t)clu_positions(f) * 4 + npiv + 16;
+__host__ __device__ __forceinline__ int clu_blocks(int npiv) { return npiv / (SB - 1) + 2; }
+__host__ __device__ __forceinline__ int clu_vector(int f, int npiv) {
+  return f > 2 * npiv ? f : 2 * npiv;
 }
-__device__ __forceinline__ CluSmem clu_smem(double* raw, int f) {
+__host__ __device__ __forceinline__ size_t clu_bytes(int f, int npiv) {
+  return ((size_t)clu_vector(f, npiv) + 2 * DB + clu_blocks(npiv)) * 8 +
+         (size_t)clu_positions(f) * 4 + 2 * (size_t)clu_blocks(npiv) + npiv + 16;
+}
+__device__ __forceinline__ CluSmem clu_smem(double* raw, int f, int npiv) {
   CluSmem m;
   m.V = raw;
-  m.part = raw + f;
-  m.diag = m.part + NT;
-  m.P = reinterpret_cast<int*>(m.diag + 2 * DB);
-  m.K = reinterpret_cast<unsigned char*>(m.P + clu_positions(f));
+  m.diag = raw + clu_vector(f, npiv);
+  m.bar = reinterpret_cast<unsigned long long*>(m.diag + 2 * DB);
+  m.P = reinterpret_cast<int*>(m.bar + clu_blocks(npiv));
+  m.jb = reinterpret_cast<unsigned short*>(m.P + clu_positions(f));
+  m.K = reinterpret_cast<unsigned char*>(m.jb + clu_blocks(npiv));
   return m;
 }
-// The diagonal block of columns [jb, je) into `dst` (in flight until cp_wait);
-// T entries, leading dimension SB + 1.
+
+// The diagonal block of columns [jb, jb + bw) into `dst` (in flight until
+// cp_wait); T entries, leading dimension SB + 1.
 template <class T>
 __device__ __forceinline__ void fetch_diag(const T* L, int f, int jb, int bw, double* dst) {
   T* o = reinterpret_cast<T*>(dst);
@@ -581,33 +592,70 @@ __device__ __forceinline__ void fetch_diag(const T* L, int f, int jb, int bw, do
       if (i >= j) cp_async_el(o + i + j * (SB + 1), L + jb + i + (size_t)(jb + j) * f);
 }
 
-// CTA 0's part is a chain of 32-column blocks: the block's diagonal is in
-// shared memory and its entries of the next 256 rows in registers before its
-// turn comes (loaded while the previous block is solved and applied), so a
-// block costs the warp's triangular solve and 32 multiply-adds a row, without
-// a global load in between.  One solve of the 2D SIMP 128x64 KKT (fronts of
-// ~1,100 rows and ~280 pivots, one after another) 3.77 -> 2.44 ms.
+// Pivot kinds and blocks of a front (every CTA), and its mbarriers; returns
+// the number of blocks.  forward: blocks from the first column on (block_end),
+// else from the last one backwards.
+__device__ __forceinline__ int clu_setup(const CluSmem& m, const int* kind, int npiv,
+                                         bool forward, int* s_nb) {
+  const int tid = threadIdx.x;
+  for (int j = tid; j < npiv; j += NT) m.K[j] = (unsigned char)kind[j];
+  for (int b = tid; b < clu_blocks(npiv); b += NT) msg::init(m.bar + b);
+  msg::init_done();
+  __syncthreads();
+  if (tid == 0) {
+    // first columns in the order of the sweep, then its end
+    int nb = 0, j = forward ? 0 : npiv;
+    while (forward ? j < npiv : j > 0) {
+      m.jb[nb++] = (unsigned short)j;
+      if (forward) {
+        int je = min(j + SB, npiv);
+        if (je < npiv && m.K[je - 1] == 1) je++;
+        j = je;
+      } else {
+        int jb = max(j - SB, 0);
+        if (jb > 0 && m.K[jb] == 2) jb--;  // keep 2x2 pairs together
+        j = jb;
+      }
+    }
+    m.jb[nb] = (unsigned short)j;
+    *s_nb = nb;
+  }
+  __syncthreads();
+  return *s_nb;
+}
+
+// CTA 0 carries the pivot chain: a block's diagonal is in shared memory and its
+// entries of the next 256 rows in registers before its turn comes, so a block
+// costs one warp's triangular solve and 32 multiply-adds a row, without a global
+// load in between.  The other seven CTAs hold the rows below the pivots; CTA 0
+// sends them each block's solution as messages (cluster_msg.cuh), so they work
+// on a block while CTA 0 is at the next and no cluster barrier stands between
+// blocks (405 cycles each, 935 after remote stores).  One solve of the 2D SIMP
+// 128x64 KKT (fronts of ~1,100 rows and ~280 pivots, one after another): 3.77 ms
+// with every CTA's entries fetched from global memory at its turn, 2.44 with the
+// fetches ahead and a cluster barrier a block, 2.02 with the messages.
 template <class T>
 __global__ void __launch_bounds__(NT, 1)
-k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
-              int nrhs, int ldx, double* ubuf, const long long* uoff) {
-  pdl_enter();
+k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs, int ldx,
+              double* ubuf, const long long* uoff, int* err) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double sm[];
+  __shared__ int s_nb;
+  __shared__ int s_kid[kCluKids], s_cc[kCluKids];
+  __shared__ long long s_uc[kCluKids];
   const int cr = (int)cluster.block_rank();
   const int node = nodes[blockIdx.x / CS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NWARP = NT / 32;
   const int f = d.f[node], npiv = d.npiv[node];
   const int* fvars = d.ipool + d.ioff[node];
-  const int* kind = fvars + 3 * f;
   const T* L = reinterpret_cast<const T*>(d.fpool) + d.foff[node];
-  const CluSmem m = clu_smem(sm, f);
+  const CluSmem m = clu_smem(sm, f, npiv);
   double* V = m.V;
   const int ns = d.ns[node], ndin = d.ndin[node], fs = ns + ndin;
   const int* fsinv = fvars + 2 * f;
-  const int q0 = d.kid_ptr[node], q1 = d.kid_ptr[node + 1];
+  const int q0 = d.kid_ptr[node], nk = d.kid_ptr[node + 1] - q0;
+  const int nb = clu_setup(m, fvars + 3 * f, npiv, true, &s_nb);
   auto position = [&](int c, int ndc, int choff, int a) {
     int pos;
     if (a < ndc) {
@@ -618,61 +666,103 @@ k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
     }
     return pos < fs ? fsinv[pos] : pos;
   };
-  int held = 0;
+  int held = 0;  // children whose rows' positions are held
+  const int vb = d.var_ptr[node];
   if (cr == 0) {
-    for (int j = tid; j < npiv; j += NT) m.K[j] = (unsigned char)kind[j];
-    for (int q = q0, choff = ns, at = 0; q < q1; q++) {
-      const int c = d.kids[q], ndc = d.ndel[c], cc = d.f[c] - d.npiv[c];
+    if (tid < min(nk, kCluKids)) {
+      const int c = d.kids[q0 + tid];
+      s_kid[tid] = c;
+      s_cc[tid] = d.f[c] - d.npiv[c];
+      s_uc[tid] = uoff[c];
+    }
+    for (int q = 0, choff = ns, at = 0; q < min(nk, kCluKids); q++) {
+      const int c = d.kids[q0 + q], ndc = d.ndel[c], cc = d.f[c] - d.npiv[c];
       if (at + cc > clu_positions(f)) break;
       for (int a = tid; a < cc; a += NT) m.P[at + a] = position(c, ndc, choff, a);
       at += cc;
       choff += ndc;
-      held = q + 1 - q0;
+      held = q + 1;
     }
   }
+  // the other CTAs' rows: 32-row strips dealt over them, a row a thread (and
+  // every 256th after it)
+  const int nstrip = (f - npiv + 31) / 32;
+  auto row_of = [&](int t) { return npiv + ((cr - 1) + CW * (t >> 5)) * 32 + (t & 31); };
+  const int nrow = cr > 0 ? 32 * ((nstrip - (cr - 1) + CW - 1) / CW) : 0;
+  if (cr > 0)
+    for (int b = tid; b < nb; b += NT)
+      msg::expect(m.bar + b, 8u * (unsigned)(m.jb[b + 1] - m.jb[b]));
+  // the columns' products are summed in eight segments, added in order
+  const int seg = (npiv + 7) / 8;
+  cluster.sync();
+  pdl_enter();
+  unsigned phase = 0;
   for (int rhs = blockIdx.y; rhs < nrhs; rhs += gridDim.y) {
     double* G = ubuf + uoff[node] + (long long)rhs * f;
     double* xr = x + (long long)rhs * ldx;
     if (cr == 0) {
       for (int r = tid; r < f; r += NT) V[r] = 0.0;
+      if (nb > 0) fetch_diag<T>(L, f, 0, m.jb[1], m.diag);
       __syncthreads();
-      const int vb = d.var_ptr[node];
       for (int r = tid; r < ns; r += NT) V[fsinv[r]] = xr[d.vars[vb + r]];
       __syncthreads();
-      auto end_of = [&](int jb) {
-        int je = min(jb + SB, npiv);
-        if (je < npiv && m.K[je - 1] == 1) je++;
-        return je;
-      };
-      int jb = 0, je = npiv > 0 ? end_of(0) : 0, buf = 0;
-      fetch_diag<T>(L, f, 0, je, m.diag);
-      for (int q = q0, choff = ns, at = 0; q < q1; q++) {
-        const int c = d.kids[q], ndc = d.ndel[c], npc = d.npiv[c], cc = d.f[c] - npc;
-        const double* uc = ubuf + uoff[c] + (long long)rhs * d.f[c] + npc;
-        const bool in_p = q - q0 < held;
+      for (int q = 0, choff = ns, at = 0; q < nk; q++) {
+        const int c = q < kCluKids ? s_kid[q] : d.kids[q0 + q];
+        const int cc = q < kCluKids ? s_cc[q] : d.f[c] - d.npiv[c];
+        const double* uc = ubuf + (q < kCluKids ? s_uc[q] : uoff[c]) +
+                           (long long)rhs * d.f[c] + d.npiv[c];
+        const int ndc = d.ndel[c];
         for (int a = tid; a < cc; a += NT)
-          V[in_p ? m.P[at + a] : position(c, ndc, choff, a)] += __ldcg(uc + a);
+          V[q < held ? m.P[at + a] : position(c, ndc, choff, a)] += __ldcg(uc + a);
         __syncthreads();
         at += cc;
         choff += ndc;
       }
-      while (jb < npiv) {
-        const int bw = je - jb;
-        // the block's entries of this thread's row, its 33rd column apart
-        const int i0 = je + tid;
-        const T* Li = L + (i0 < npiv ? i0 : 0) + (size_t)jb * f;
-        T a[SB];
-#pragma unroll
-        for (int j = 0; j < SB; j++) a[j] = i0 < npiv && j < bw ? Li[(size_t)j * f] : T(0);
-        const T a32 = i0 < npiv && bw > SB ? Li[(size_t)SB * f] : T(0);
+      for (int b = 0; b < nb; b++) {
+        const int jb = m.jb[b], je = m.jb[b + 1], bw = je - jb;
+        const T* D = reinterpret_cast<const T*>(m.diag + (b & 1) * DB);
+        // warp 0 solves; the other warps load the block's entries of the next
+        // 224 rows (a row a thread, the 33rd column apart) and the next
+        // diagonal block meanwhile
+        const int i0 = warp > 0 ? je + tid - 32 : npiv;
+        T a[SB], a32 = T(0);
         cp_wait();
         __syncthreads();  // the diagonal block; the rows' updates of the last one
-        if (warp == 0)
-          lower_block<T>(reinterpret_cast<const T*>(m.diag + buf * DB), SB + 1, m.K + jb, bw,
-                         V + jb, lane);
-        const int jn = je < npiv ? end_of(je) : je;
-        if (je < npiv) fetch_diag<T>(L, f, je, jn - je, m.diag + (buf ^ 1) * DB);
+        if (warp == 0) {
+          lower_block<T>(D, SB + 1, m.K + jb, bw, V + jb, lane);
+        } else {
+          const T* Li = L + (i0 < npiv ? i0 : 0) + (size_t)jb * f;
+#pragma unroll
+          for (int j = 0; j < SB; j++) a[j] = i0 < npiv && j < bw ? Li[(size_t)j * f] : T(0);
+          if (bw > SB && i0 < npiv) a32 = Li[(size_t)SB * f];
+        }
+        if (b + 1 < nb)
+          fetch_diag<T>(L, f, je, m.jb[b + 2] - je, m.diag + ((b + 1) & 1) * DB);
         __syncthreads();
+        if (warp == NT / 32 - 1 && nstrip > 0) {
+          // the block's values to the other CTAs
+          for (int j = lane; j < bw; j += 32)
+#pragma unroll
+            for (int r = 1; r < CS; r++)
+              msg::send(msg::remote(V + jb + j, r), msg::remote(m.bar + b, r), V[jb + j]);
+        }
+        if (warp == NT / 32 - 2) {
+          // D^{-1} and the pivots' forward values
+          for (int j = lane; j < bw; j += 32) {
+            const int kd = m.K[jb + j];
+            double v;
+            if (kd == 0) {
+              v = V[jb + j] / (double)D[j * (SB + 2)];
+            } else {
+              const T* Df = D + (j - kd + 1) * (SB + 2);  // the pair's first diagonal
+              const double d11 = Df[0], d21 = Df[1], d22 = Df[SB + 2];
+              const double inv = inv2x2(d11, d21, d22);
+              v = kd == 1 ? piv2_first(inv, d21, d22, V[jb + j], V[jb + j + 1])
+                          : piv2_second(inv, d11, d21, V[jb + j - 1], V[jb + j]);
+            }
+            xr[decode_var(fvars[jb + j])] = v;
+          }
+        }
         if (i0 < npiv) {
           double acc = 0.0;
 #pragma unroll
@@ -681,150 +771,193 @@ k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
           if (bw > SB) acc = __fma_rn((double)a32, V[jb + SB], acc);
           V[i0] -= acc;
         }
-        for (int i = i0 + NT; i < npiv; i += NT)
+        for (int i = je + tid + NT - 32; i < npiv; i += NT)
           V[i] -= dot_strided(L + i + (size_t)jb * f, (size_t)f, bw,
                               [&](int j) { return V[jb + j]; });
-        jb = je;
-        je = jn;
-        buf ^= 1;
       }
-      __syncthreads();
-      for (int t = tid; t < f; t += NT) G[t] = V[t];
-    }
-    cluster.sync();
-    // contribution rows: G[i] -= L21[i, :] y1, 32-row strips over the
-    // cluster's CTAs, the pivot columns split over the CTA's warps and the
-    // warps' partial sums added in a fixed order
-    if (cr != 0) copy_cg(V, G, npiv);
-    __syncthreads();
-    const int ncr = f - npiv;
-    const int nstrip = (ncr + 31) / 32;
-    const int jc = (npiv + NWARP - 1) / NWARP;
-    const int j0 = warp * jc, j1 = min(npiv, j0 + jc);
-    for (int st = cr; st < nstrip; st += CS) {
-      const int i = npiv + st * 32 + lane;
-      double acc = 0.0;
-      if (i < f && j1 > j0)
-        acc = dot_strided(L + i + (size_t)j0 * f, (size_t)f, j1 - j0,
-                          [&](int j) { return V[j0 + j]; });
-      m.part[warp * 32 + lane] = acc;
-      __syncthreads();
-      if (warp == 0 && i < f) {
-        double s = 0.0;
-        for (int w = 0; w < NWARP; w++) s += m.part[w * 32 + lane];
-        G[i] = __ldcg(G + i) - s;
+    } else if (nstrip > 0) {
+      // G[i] -= L21[i, :] y1: s and acc of this thread's first row in
+      // registers, of its other rows behind the pivots' values
+      double s0 = 0.0, acc0 = 0.0;
+      double* more = V + npiv;
+      for (int t = tid + NT; t < nrow; t += NT) {
+        more[2 * (t - NT)] = 0.0;
+        more[2 * (t - NT) + 1] = 0.0;
       }
-      __syncthreads();
-    }
-    // D^{-1} and the pivots' values (CTA 0, from its shared copy)
-    if (cr == 0) {
-      for (int j = tid; j < npiv; j += NT) {
-        const int kd = m.K[j];
-        double v;
-        if (kd == 0) {
-          v = V[j] / (double)L[j + (size_t)j * f];
-        } else {
-          const T* Lf = L + (j - kd + 1) * ((size_t)f + 1);  // the pair's first diagonal
-          const double d11 = Lf[0], d21 = Lf[1], d22 = Lf[f + 1];
-          const double inv = inv2x2(d11, d21, d22);
-          v = kd == 1 ? piv2_first(inv, d21, d22, V[j], V[j + 1])
-                      : piv2_second(inv, d11, d21, V[j - 1], V[j]);
+      const int i0 = row_of(tid);
+      const bool on = tid < nrow && i0 < f;
+      for (int b = 0; b < nb; b++) {
+        const int jb = m.jb[b], bw = m.jb[b + 1] - jb;
+        const T* Li = L + (on ? i0 : npiv) + (size_t)jb * f;
+        T a[SB];
+#pragma unroll
+        for (int j = 0; j < SB; j++) a[j] = on && j < bw ? Li[(size_t)j * f] : T(0);
+        const T a32 = on && bw > SB ? Li[(size_t)SB * f] : T(0);
+        msg::wait(m.bar + b, phase, err, kCluWait);
+        int left = seg - jb % seg;  // columns to the end of the segment
+        auto add = [&](double v, int j, double& s, double& acc, int& rest) {
+          acc = __fma_rn(v, V[jb + j], acc);
+          if (--rest == 0) {
+            s += acc;
+            acc = 0.0;
+            rest = seg;
+          }
+        };
+        int rest = left;
+#pragma unroll
+        for (int j = 0; j < SB; j++)
+          if (j < bw) add((double)a[j], j, s0, acc0, rest);
+        if (bw > SB) add((double)a32, SB, s0, acc0, rest);
+        for (int t = tid + NT; t < nrow; t += NT) {
+          const int i = row_of(t);
+          if (i >= f) break;
+          const T* Lt = L + i + (size_t)jb * f;
+          double s = more[2 * (t - NT)], acc = more[2 * (t - NT) + 1];
+          rest = left;
+          for (int j = 0; j < bw; j += 16) {
+            T e[16];
+#pragma unroll
+            for (int u = 0; u < 16; u++) e[u] = j + u < bw ? Lt[(size_t)(j + u) * f] : T(0);
+#pragma unroll
+            for (int u = 0; u < 16; u++)
+              if (j + u < bw) add((double)e[u], j + u, s, acc, rest);
+          }
+          more[2 * (t - NT)] = s;
+          more[2 * (t - NT) + 1] = acc;
         }
-        xr[decode_var(fvars[j])] = v;
+      }
+      if (npiv % seg != 0) {
+        s0 += acc0;
+        for (int t = tid + NT; t < nrow; t += NT)
+          more[2 * (t - NT)] += more[2 * (t - NT) + 1];
+      }
+      // (armed again for the next right-hand side; the barrier below comes
+      // before CTA 0 sends it)
+      __syncthreads();
+      for (int b = tid; b < nb; b += NT)
+        msg::expect(m.bar + b, 8u * (unsigned)(m.jb[b + 1] - m.jb[b]));
+      acc0 = s0;
+      cluster.sync();
+      const double* V0 = cluster.map_shared_rank(V, 0);
+      if (on) G[i0] = V0[i0] - acc0;
+      for (int t = tid + NT; t < nrow; t += NT) {
+        const int i = row_of(t);
+        if (i < f) G[i] = V0[i] - more[2 * (t - NT)];
       }
     }
-    cluster.sync();
+    if (cr == 0 || nstrip == 0) cluster.sync();
+    phase ^= 1u;
+    cluster.sync();  // CTA 0's vector has been read
   }
 }
 
 template <class T>
 __global__ void __launch_bounds__(NT, 1)
-k_clu_backward(DevicePlan d, const int* __restrict__ nodes, double* x,
-               int nrhs, int ldx, double* ubuf, const long long* uoff) {
-  pdl_enter();
+k_clu_backward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs, int ldx,
+               double* ubuf, const long long* uoff, int* err) {
+  (void)ubuf;
+  (void)uoff;
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double sm[];
+  __shared__ int s_nb;
   const int cr = (int)cluster.block_rank();
   const int node = nodes[blockIdx.x / CS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NWARP = NT / 32;
   const int f = d.f[node], npiv = d.npiv[node];
   const int* fvars = d.ipool + d.ioff[node];
-  const int* kind = fvars + 3 * f;
   const T* L = reinterpret_cast<const T*>(d.fpool) + d.foff[node];
   const int ncr = f - npiv;
-  const CluSmem m = clu_smem(sm, f);
-  double* sx = m.V + npiv;    // contribution rows' final values
-  double* V = m.V;            // CTA 0: pivot values
-  if (cr == 0)
-    for (int j = tid; j < npiv; j += NT) m.K[j] = (unsigned char)kind[j];
+  const CluSmem m = clu_smem(sm, f, npiv);
+  double* V = m.V;            // CTA 0: pivot values, then the columns' corrections
+  double* sx = m.V;           // the other CTAs: contribution rows' final values
+  const int nb = clu_setup(m, fvars + 3 * f, npiv, false, &s_nb);
+  double* cor = V + npiv;
+  const bool rows = ncr > 0;
+  if (cr == 0 && rows)
+    for (int b = tid; b < nb; b += NT)
+      msg::expect(m.bar + b, 8u * (unsigned)(m.jb[b] - m.jb[b + 1]));
+  cluster.sync();
+  pdl_enter();
+  unsigned phase = 0;
   for (int rhs = blockIdx.y; rhs < nrhs; rhs += gridDim.y) {
-    double* G = ubuf + uoff[node] + (long long)rhs * f;
     double* xr = x + (long long)rhs * ldx;
-    for (int r = tid; r < ncr; r += NT) sx[r] = xr[fvars[npiv + r]];
-    __syncthreads();
-    // t[j] = z[j] - L21[:, j]^T x2 for every pivot column, one warp per
-    // column over the cluster's warps
-    for (int j = cr * NWARP + warp; j < npiv; j += CS * NWARP) {
-      const double acc = warp_sum_down(lane_dot(L + (size_t)j * f + npiv, 0, ncr, lane,
-                                                [&](int i) { return sx[i]; }));
-      if (lane == 0) G[j] = xr[decode_var(fvars[j])] - acc;
+    // t[j] = z[j] - L21[:, j]^T x2 for every pivot column, one warp per column
+    // over the other CTAs' warps, the last columns first
+    if (cr > 0 && rows) {
+      for (int r = tid; r < ncr; r += NT) sx[r] = xr[fvars[npiv + r]];
+      __syncthreads();
+      int b = 0;
+      for (int o = (cr - 1) * NWARP + warp; o < npiv; o += CW * NWARP) {
+        const int j = npiv - 1 - o;
+        while (m.jb[b + 1] > j) b++;
+        const double acc = warp_sum_down(lane_dot(L + (size_t)j * f + npiv, 0, ncr, lane,
+                                                  [&](int i) { return sx[i]; }));
+        if (lane == 0)
+          msg::send(msg::remote(cor + j, 0), msg::remote(m.bar + b, 0), acc);
+      }
     }
-    cluster.sync();
     if (cr == 0) {
-      for (int t = tid; t < npiv; t += NT) V[t] = __ldcg(G + t);
-      auto begin_of = [&](int je) {
-        int jb = max(je - SB, 0);
-        if (jb > 0 && m.K[jb] == 2) jb--;  // keep 2x2 pairs together
-        return jb;
-      };
-      int je = npiv, jb = npiv > 0 ? begin_of(npiv) : 0, buf = 0;
-      if (npiv > 0) fetch_diag<T>(L, f, jb, je - jb, m.diag);
-      while (je > 0) {
-        // t[j] -= sum_{je <= i < npiv} L[i, j] t[i] for j in [jb, je): four or
-        // five columns a warp together, the entries of the rows that do not
-        // wait for the last block loaded before it was done
-        constexpr int CW = (SB + 1 + NWARP - 1) / NWARP, RW = 8;
-        const int jw = jb + warp;  // this warp's columns: jw, jw + NWARP, ...
-        T pre[CW][RW];
+      if (nb > 0) fetch_diag<T>(L, f, m.jb[1], m.jb[0] - m.jb[1], m.diag);
+      for (int t = tid; t < npiv; t += NT) V[t] = xr[decode_var(fvars[t])];
+      // columns jb + (warp - 1) + 7 u of a block are warp's (1 .. 7); their
+      // entries of the first 256 rows below the block are loaded while warp 0
+      // solves the block before
+      constexpr int NW1 = NWARP - 1, CWP = (SB + 1 + NW1 - 1) / NW1, RW = 8;
+      T pre[CWP][RW];
+      auto load_pre = [&](int jb, int je) {
 #pragma unroll
-        for (int u = 0; u < CW; u++)
+        for (int u = 0; u < CWP; u++)
 #pragma unroll
           for (int r = 0; r < RW; r++) {
-            const int j = jw + NWARP * u, i = je + lane + 32 * r;
+            const int j = jb + warp - 1 + NW1 * u, i = je + lane + 32 * r;
             pre[u][r] = j < je && i < npiv ? L[i + (size_t)j * f] : T(0);
           }
-        __syncthreads();  // the last block's values
-#pragma unroll
-        for (int u = 0; u < CW; u++) {
-          const int j = jw + NWARP * u;
-          if (j >= je) break;
-          double acc = 0.0;
-#pragma unroll
-          for (int r = 0; r < RW; r++) {
-            const int i = je + lane + 32 * r;
-            if (i < npiv) acc = __fma_rn((double)pre[u][r], V[i], acc);
-          }
-          for (int i = je + lane + 32 * RW; i < npiv; i += 32)
-            acc = __fma_rn((double)L[i + (size_t)j * f], V[i], acc);
-          acc = warp_sum_down(acc);
-          if (lane == 0) V[j] -= acc;
-        }
+      };
+      if (warp > 0 && nb > 0) load_pre(m.jb[1], m.jb[0]);
+      for (int b = 0; b < nb; b++) {
+        const int je = m.jb[b], jb = m.jb[b + 1];
+        if (rows) msg::wait(m.bar + b, phase, err, kCluWait);
         cp_wait();
+        __syncthreads();  // the last block's values
+        // t[j] -= sum_{je <= i < npiv} L[i, j] t[i] for j in [jb, je)
+        if (warp > 0) {
+#pragma unroll
+          for (int u = 0; u < CWP; u++) {
+            const int j = jb + warp - 1 + NW1 * u;
+            if (j < je) {
+              double acc = 0.0;
+#pragma unroll
+              for (int r = 0; r < RW; r++) {
+                const int i = je + lane + 32 * r;
+                if (i < npiv) acc = __fma_rn((double)pre[u][r], V[i], acc);
+              }
+              for (int i = je + lane + 32 * RW; i < npiv; i += 32)
+                acc = __fma_rn((double)L[i + (size_t)j * f], V[i], acc);
+              acc = warp_sum_down(acc);
+              if (lane == 0) V[j] = (rows ? V[j] - cor[j] : V[j]) - acc;
+            }
+          }
+        }
         __syncthreads();
         if (warp == 0)
-          upper_block<T>(reinterpret_cast<const T*>(m.diag + buf * DB), SB + 1, m.K + jb,
+          upper_block<T>(reinterpret_cast<const T*>(m.diag + (b & 1) * DB), SB + 1, m.K + jb,
                          je - jb, V + jb, lane);
-        const int jn = jb > 0 ? begin_of(jb) : 0;
-        if (jb > 0) fetch_diag<T>(L, f, jn, jb - jn, m.diag + (buf ^ 1) * DB);
-        je = jb;
-        jb = jn;
-        buf ^= 1;
+        else if (b + 1 < nb)
+          load_pre(m.jb[b + 2], jb);
+        if (b + 1 < nb)
+          fetch_diag<T>(L, f, m.jb[b + 2], jb - m.jb[b + 2], m.diag + ((b + 1) & 1) * DB);
       }
       __syncthreads();
       for (int j = tid; j < npiv; j += NT) xr[decode_var(fvars[j])] = V[j];
+      // (armed again for the next right-hand side; the barrier below comes
+      // before its corrections are sent)
+      if (rows)
+        for (int b = tid; b < nb; b += NT)
+          msg::expect(m.bar + b, 8u * (unsigned)(m.jb[b] - m.jb[b + 1]));
     }
+    phase ^= 1u;
     cluster.sync();
   }
 }
@@ -1135,7 +1268,8 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block,
 template <class K>
 static int launch_cluster(K kernel, int fronts, int smem, cudaStream_t s,
                           const DevicePlan& d, const int* nodes, double* x,
-                          int nrhs, int ldx, double* ubuf, const long long* uoff) {
+                          int nrhs, int ldx, double* ubuf, const long long* uoff,
+                          int* err) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(fronts * CS, std::max(1, std::min(nrhs, kRhsSlices)));
   cfg.blockDim = dim3(NT);
@@ -1150,7 +1284,7 @@ static int launch_cluster(K kernel, int fronts, int smem, cudaStream_t s,
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  SCUDA(cudaLaunchKernelEx(&cfg, kernel, d, nodes, x, nrhs, ldx, ubuf, uoff));
+  SCUDA(cudaLaunchKernelEx(&cfg, kernel, d, nodes, x, nrhs, ldx, ubuf, uoff, err));
   ab::count_launch();
   return 0;
 }
@@ -1250,7 +1384,13 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
                              (int)nodes.size() - h.sv_wide_ptr[l]);
   }
   h.sv_narrow_ptr[L] = h.sv_clu_ptr[L] = h.sv_wide_ptr[L] = (int)nodes.size();
-  if (!h.sv_nodes) SCUDA(cudaMalloc((void**)&h.sv_nodes, std::max(nn, 1) * sizeof(int)));
+  if (!h.sv_nodes) {
+    SCUDA(cudaMalloc((void**)&h.sv_nodes, std::max(nn, 1) * sizeof(int)));
+    SCUDA(cudaMalloc((void**)&h.sv_ctr, (kEpochWord + 1) * sizeof(unsigned)));
+    SCUDA(cudaMalloc((void**)&h.sv_err, sizeof(int)));
+    SCUDA(cudaMemsetAsync(h.sv_ctr, 0, (kEpochWord + 1) * sizeof(unsigned), s));
+    SCUDA(cudaMemsetAsync(h.sv_err, 0, sizeof(int), s));
+  }
   if (h.sv_max_wide > h.sv_state_cap) {
     if (h.sv_state) SCUDA(cudaFree(h.sv_state));
     h.sv_state = nullptr;
@@ -1290,12 +1430,8 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
       SCUDA(cudaMalloc((void**)&h.sv_dep, std::max(nn, 1) * sizeof(int)));
       SCUDA(cudaMalloc((void**)&h.sv_done,
                        2 * kRhsSlices * (size_t)std::max(nn, 1) * sizeof(unsigned)));
-      SCUDA(cudaMalloc((void**)&h.sv_ctr, (kEpochWord + 1) * sizeof(unsigned)));
-      SCUDA(cudaMalloc((void**)&h.sv_err, sizeof(int)));
       SCUDA(cudaMemsetAsync(h.sv_done, 0,
                             2 * kRhsSlices * (size_t)std::max(nn, 1) * sizeof(unsigned), s));
-      SCUDA(cudaMemsetAsync(h.sv_ctr, 0, (kEpochWord + 1) * sizeof(unsigned), s));
-      SCUDA(cudaMemsetAsync(h.sv_err, 0, sizeof(int), s));
     }
     SCUDA(cudaMemcpyAsync(h.sv_bq, bq.data(), qc * sizeof(int), cudaMemcpyHostToDevice, s));
     SCUDA(cudaMemcpyAsync(h.sv_dep, dep.data(), qc * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -1402,6 +1538,10 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
   const int qsm = h.sv_qsmem;
   const unsigned* ep = h.sv_ctr + kEpochWord;   // this solve's epoch, set on the device
   const int slices = std::max(1, std::min(nrhs, kRhsSlices));
+  // (without a programmatic launch of its own it starts after everything before
+  // it is done: the launches that follow read the factor ahead of their turn)
+  { k_sweep_begin<<<1, 32, 0, s>>>(h.sv_ctr); ab::count_launch(); }
+  SCUDA(cudaGetLastError());
   if (queue) {
     if (h.sv_qgrid == 0 || h.sv_qgrid_small != qsmall) {
       // CTAs resident at once, at most one per queued front
@@ -1417,8 +1557,6 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
       h.sv_qgrid = std::max(1, std::min(h.sv_qcount, sms * std::max(per, 1)));
       h.sv_qgrid_small = qsmall;
     }
-    { k_sweep_begin<<<1, 32, 0, s>>>(h.sv_ctr); ab::count_launch(); }
-    SCUDA(cudaGetLastError());
     if (qsmall)
       SCUDA(launch_pdl(k_solve_forward_q<T, kSmallThreads>, dim3(h.sv_qgrid, slices), dim3(qth),
                        (size_t)qsm, s, d, (const int*)h.sv_nodes, h.sv_qcount, d_x, nrhs,
@@ -1452,7 +1590,7 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
     const int cb = h.sv_clu_ptr[l], ccnt = h.sv_wide_ptr[l] - cb;
     if (ccnt) {
       int rc = launch_cluster(k_clu_forward<T>, ccnt, h.sv_clu_smem[l], s, d,
-                              h.sv_nodes + cb, d_x, nrhs, ldx, h.ubuf, h.uoff);
+                              h.sv_nodes + cb, d_x, nrhs, ldx, h.ubuf, h.uoff, h.sv_err);
       if (rc) return rc;
     }
     const int wb = h.sv_wide_ptr[l], wc = h.sv_narrow_ptr[l + 1] - wb;
@@ -1491,7 +1629,7 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
     const int cb = h.sv_clu_ptr[l], ccnt = h.sv_wide_ptr[l] - cb;
     if (ccnt) {
       int rc = launch_cluster(k_clu_backward<T>, ccnt, h.sv_clu_smem[l], s, d,
-                              h.sv_nodes + cb, d_x, nrhs, ldx, h.ubuf, h.uoff);
+                              h.sv_nodes + cb, d_x, nrhs, ldx, h.ubuf, h.uoff, h.sv_err);
       if (rc) return rc;
     }
     const int wb = h.sv_wide_ptr[l], wc = h.sv_narrow_ptr[l + 1] - wb;

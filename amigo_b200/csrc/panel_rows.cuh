@@ -32,16 +32,6 @@ constexpr int kRowThreads = 256;
 
 constexpr int kRowMoves = 16;  // positions moved per flush
 
-// What a warp keeps, and a CTA sends to the others, in a reduction: the bits
-// of the largest |candidate entry| (h, l) and its position i (kNoPos: none),
-// those of the largest |other entry| (th, tl), and a value of the row the
-// step is about (wh, wl).  Non-negative doubles order like their bits, so the
-// folds are integer maxima (redux.sync).
-struct alignas(16) RowEntry {
-  unsigned h, l, i, th, tl, wh, wl, pad;
-};
-constexpr unsigned kNoPos = 0x7fffffffu;
-
 // Messages of a step: the reduction over the candidate column together with
 // the next candidate's W row (RED), the W row of column imax (IMAX), the
 // reduction over it (RED2), and the next candidate's W row when it was not
@@ -76,123 +66,11 @@ __device__ __forceinline__ void row_barrier() {
   }
 }
 
-// The shared-memory address of `p` in CTA r of the cluster.
-__device__ __forceinline__ unsigned row_remote(const void* p, int r) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-  unsigned d;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(r));
-  return d;
-}
-
-// First-argmax (h, l, i) and maximum (th, tl) of a warp, in every lane.
-__device__ __forceinline__ void row_fold_max(unsigned& th, unsigned& tl) {
-  const unsigned m = __reduce_max_sync(0xffffffffu, th);
-  tl = __reduce_max_sync(0xffffffffu, th == m ? tl : 0u);
-  th = m;
-}
-__device__ __forceinline__ void row_fold(RowEntry& e) {
-  const unsigned FULL = 0xffffffffu;
-  const unsigned mh = __reduce_max_sync(FULL, e.h);
-  const unsigned ml = __reduce_max_sync(FULL, e.h == mh ? e.l : 0u);
-  e.i = __reduce_min_sync(FULL, e.h == mh && e.l == ml ? e.i : kNoPos);
-  e.h = mh;
-  e.l = ml;
-  row_fold_max(e.th, e.tl);
-}
-__device__ __forceinline__ double row_bits(unsigned h, unsigned l) {
-  return __hiloint2double((int)h, (int)l);
-}
-// |a| at position p into the argmax (cand) or into the maximum (other); a NaN
-// counts as no entry.  (Selects, not branches.)
-__device__ __forceinline__ void row_argmax(RowEntry& e, double a, int p, bool cand) {
-  const unsigned h = (unsigned)__double2hiint(a), l = (unsigned)__double2loint(a);
-  const unsigned long long x = ((unsigned long long)h << 32) | l;
-  const unsigned long long y = ((unsigned long long)e.h << 32) | e.l;
-  const bool gt = cand && a == a && (x > y || (x == y && (unsigned)p < e.i));
-  e.h = gt ? h : e.h;
-  e.l = gt ? l : e.l;
-  e.i = gt ? (unsigned)p : e.i;
-}
-__device__ __forceinline__ void row_max(RowEntry& e, double a, bool other) {
-  const unsigned h = (unsigned)__double2hiint(a), l = (unsigned)__double2loint(a);
-  const unsigned long long x = ((unsigned long long)h << 32) | l;
-  const unsigned long long y = ((unsigned long long)e.th << 32) | e.tl;
-  const bool gt = other && a == a && x > y;
-  e.th = gt ? h : e.th;
-  e.tl = gt ? l : e.tl;
-}
-
-// Stores into another CTA's shared memory that report their bytes to that
-// CTA's mbarrier: no fence and no cluster barrier between the value and the
-// reader, who waits for the bytes (measured on clusters of 8: 405 cycles for
-// a release / acquire cluster barrier, 935 with one remote store per warp
-// and CTA before it).
-__device__ __forceinline__ void row_send(unsigned dst, unsigned bar, float v) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 "
-               "[%0], %1, [%2];" ::"r"(dst), "r"(__float_as_uint(v)), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void row_send(unsigned dst, unsigned bar, double v) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 "
-               "[%0], %1, [%2];" ::"r"(dst), "l"(__double_as_longlong(v)), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void row_send4(unsigned dst, unsigned bar, uint4 v) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 "
-               "[%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z),
-               "r"(v.w), "r"(bar)
-               : "memory");
-}
-
 // A value that is the same in every lane of a warp, in a form that the compiler
 // knows to be so (a warp reduction): branches on it need no reconvergence, and
 // what is computed from it stays in uniform registers.
 __device__ __forceinline__ int row_uniform(int v) {
   return __reduce_max_sync(0xffffffffu, v);
-}
-__device__ __forceinline__ unsigned row_uniform_min(unsigned v) {
-  return __reduce_min_sync(0xffffffffu, v);
-}
-
-// Message m of parity `par` will bring `bytes` (one thread of the CTA).
-template <class C>
-__device__ __forceinline__ void row_expect(C& c, int par, int m, unsigned bytes) {
-  const unsigned bar = (unsigned)__cvta_generic_to_shared(&c.bar[par][m]);
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-               "r"(bytes)
-               : "memory");
-}
-
-// Wait until message m's bytes have arrived (phase: the bits of the mbarriers'
-// phases, one per mbarrier).  The wait is bounded: when it runs out (every
-// message is sent before its receivers can need it, so only a fault elsewhere
-// could make it), ST_WAIT is set and the warp leaves the kernel; the CTA's and
-// the cluster's barriers count threads that have left as arrived, so the other
-// warps end too.
-template <class C>
-__device__ __forceinline__ void row_wait(C& c, int par, int m, unsigned& phase,
-                                         int* status) {
-  const unsigned bar = (unsigned)__cvta_generic_to_shared(&c.bar[par][m]);
-  const int bit = 4 * par + m;
-  const unsigned ph = (phase >> bit) & 1u;
-  phase ^= 1u << bit;
-  auto poll = [&]() {
-    unsigned ok;
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(ph)
-        : "memory");
-    return row_uniform_min(ok);
-  };
-  if (poll()) return;
-  for (int it = 0; it < (1 << 20); it++)
-    if (poll()) return;
-  atomicOr(status, ST_WAIT);
-  __threadfence();
-  asm volatile("exit;");
 }
 
 // The panel's L entries of a thread's rows: complete groups of eight columns
@@ -322,11 +200,8 @@ __device__ void panel_factor_rows(T* F, int ld, T* Wg, int n, bool root, int* va
   int pc = lane, pa = 0, pb = 1;
   unsigned phase = 0;
   if constexpr (CS > 1) {
-    if (tid < 8) {
-      const unsigned bar = (unsigned)__cvta_generic_to_shared(&c.bar[tid >> 2][tid & 3]);
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (tid < 8) msg::init(&c.bar[tid >> 2][tid & 3]);
+    msg::init_done();
   }
   // every CTA of the cluster has started and its mbarriers are set up before
   // anything is sent to it
@@ -334,10 +209,15 @@ __device__ void panel_factor_rows(T* F, int ld, T* Wg, int n, bool root, int* va
   // a message has arrived (CS 1: the stores of the CTA's warps are published)
   auto wait = [&](int par, int m) {
     if constexpr (CS == 1) __syncthreads();
-    else row_wait(c, par, m, phase, status);
+    else {
+      // (phase: the bits of the mbarriers' phases, one per mbarrier)
+      const int bit = 4 * par + m;
+      msg::wait(&c.bar[par][m], (phase >> bit) & 1u, status, ST_WAIT);
+      phase ^= 1u << bit;
+    }
   };
   auto expect = [&](int par, int m, unsigned bytes) {
-    if (CS > 1 && tid == 0) row_expect(c, par, m, bytes);
+    if (CS > 1 && tid == 0) msg::expect(&c.bar[par][m], bytes);
   };
   auto load_pos = [&](int p, T (&dst)[RPT]) {
     const int q = kstart + ph[p - kstart];
@@ -358,7 +238,7 @@ __device__ void panel_factor_rows(T* F, int ld, T* Wg, int n, bool root, int* va
     } else {
 #pragma unroll
       for (int t = 0; t < CS; t++)
-        row_send(row_remote(dst + lane, t), row_remote(&c.bar[par][m], t), v);
+        msg::send(msg::remote(dst + lane, t), msg::remote(&c.bar[par][m], t), v);
     }
   };
   // this CTA's entry of a reduction to every CTA (set 0: the candidate column,
@@ -394,10 +274,10 @@ __device__ void panel_factor_rows(T* F, int ld, T* Wg, int n, bool root, int* va
         e.l = (unsigned)__double2loint(v2);
       }
       if (lane < CS) {
-        const unsigned dst = row_remote(&c.ent[par][set][cr], lane);
-        const unsigned bar = row_remote(&c.bar[par][set ? ROW_RED2 : ROW_RED], lane);
-        row_send4(dst, bar, make_uint4(e.h, e.l, e.i, e.th));
-        row_send4(dst + 16, bar, make_uint4(e.tl, (unsigned)__double2hiint(v),
+        const unsigned dst = msg::remote(&c.ent[par][set][cr], lane);
+        const unsigned bar = msg::remote(&c.bar[par][set ? ROW_RED2 : ROW_RED], lane);
+        msg::send(dst, bar, make_uint4(e.h, e.l, e.i, e.th));
+        msg::send(dst + 16, bar, make_uint4(e.tl, (unsigned)__double2hiint(v),
                                             (unsigned)__double2loint(v), 0u));
       }
     }
