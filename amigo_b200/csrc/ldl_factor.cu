@@ -26,6 +26,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/amigo_b200.h"
@@ -60,9 +61,8 @@ constexpr int kSwThreads = 512;
 constexpr int kSwRows = 4;
 constexpr int kSwSmemBytes = 200 * 1024;
 constexpr int kTile = 64;
-// Right-looking small-front kernel: rows of room for delayed pivots, and
-// its block size (measured on 68-row fronts: 32 threads 11.9 ms, 64 9.7,
-// 128 8.5, 256 8.25 for one factorization of 512 cart-pole problems).
+// Small-front kernel: rows of room for delayed pivots, and its block size
+// (128 threads: 10 to 20% more time, see small_front.cuh).
 constexpr int kRlSlack = 8;
 constexpr int kRlThreads = 256;
 
@@ -829,6 +829,8 @@ __device__ void panel_factor(T* F, int ld, T* W, int ldw, int n,
   kw_ = kw;
 }
 
+#include "pivot_fold.cuh"
+
 // ---------------------------------------------------------------------------
 // Unblocked right-looking factorization for fronts held in shared memory.
 // Every pivot's rank-1 (2x2: rank-2) update is applied to the trailing
@@ -1188,7 +1190,7 @@ __device__ __forceinline__ int child_row_pos(const DevicePlan& d, int cb,
 // pivot was accepted (0: 1x1, 1/2: first/second column of a 2x2 block),
 // plus the inverse of the fully-summed permutation used by the solves.
 template <class T>
-__device__ void finish_front(const DevicePlan& d, int node, const T* F,
+__device__ void finish_front(const DevicePlan& d, int node, const T* F, int ld,
                              int f, int fs, int npiv, int* fvars) {
   __shared__ int s_pos, s_neg;
   const int tid = threadIdx.x;
@@ -1205,11 +1207,11 @@ __device__ void finish_front(const DevicePlan& d, int node, const T* F,
   for (int j = tid; j < npiv; j += blockDim.x) {
     const int kd = kind[j];
     if (kd == 0) {
-      if ((double)F[j + (size_t)j * f] >= 0.0) pos++; else neg++;
+      if ((double)F[j + (size_t)j * ld] >= 0.0) pos++; else neg++;
     } else if (kd == 1) {
-      const double d11 = F[j + (size_t)j * f];
-      const double d21 = F[j + 1 + (size_t)j * f];
-      const double d22 = F[j + 1 + (size_t)(j + 1) * f];
+      const double d11 = F[j + (size_t)j * ld];
+      const double d21 = F[j + 1 + (size_t)j * ld];
+      const double d22 = F[j + 1 + (size_t)(j + 1) * ld];
       const double det = d11 * d22 - d21 * d21;
       if (det >= 0.0) {
         if (d11 >= 0.0) pos += 2; else neg += 2;
@@ -1297,20 +1299,22 @@ __device__ void assemble_front(const DevicePlan& d, int node, T* F, int f,
   }
 }
 
-// Small fronts with the unblocked right-looking factorization: the front
-// and its four integer sections (variables, fully-summed permutation,
-// inverse permutation, pivot kinds) in shared memory when they fit, else in
-// the pools; `smem_bytes` is the dynamic shared memory of the launch.
-// Four CTAs per SM (64 registers a thread at 256 threads): as many fronts
-// as shared memory holds for 70-row fronts.
+#include "small_front.cuh"
+
+// Small fronts: the front and its four integer sections (variables,
+// fully-summed permutation, inverse permutation, pivot kinds) in shared memory
+// (small_front.cuh); a front that delayed pivots made too large for it runs
+// factor_front_rl on the pools.  `smem_bytes` is the dynamic shared memory of
+// the launch.
 template <class T, int BT>
-__global__ void __launch_bounds__(BT, 4)
+__global__ void __launch_bounds__(BT, 1024 / BT)
 k_factor_level_rl(DevicePlan d, const int* __restrict__ nodes, int count,
                   const double* __restrict__ vals, double ustab,
                   double pivot_tol, int smem_bytes) {
   extern __shared__ double smem_raw[];
   __shared__ CtlT<BT> ctl;
   __shared__ RedSlots<BT> rs;
+  __shared__ SmallCtl sc;
   const int tid = threadIdx.x;
   const int node = nodes[blockIdx.x];
   if (!setup_front<T, BT>(d, node, ctl)) return;
@@ -1318,25 +1322,40 @@ k_factor_level_rl(DevicePlan d, const int* __restrict__ nodes, int count,
   const int f = ctl.f, fs = ctl.fs, ns = ctl.ns, ndin = ctl.ndin;
   int* fvars = d.ipool + ctl.ioff;
   T* Fg = pool + ctl.foff;
-  const long long fbytes = ((long long)f * f * (long long)sizeof(T) + 15) & ~15ll;
-  const bool in_smem = fbytes + 5ll * f * (long long)sizeof(int) <= smem_bytes;
-  T* F = in_smem ? reinterpret_cast<T*>(smem_raw) : Fg;
-  int* iv = in_smem ? reinterpret_cast<int*>(reinterpret_cast<char*>(smem_raw) + fbytes)
-                    : fvars;
-  // scratch for the child row map: shared memory, or the front's W area
-  int* rmap = in_smem ? iv + 4 * f : reinterpret_cast<int*>(Fg + (size_t)f * f);
-  if (in_smem)
+  if (small_bytes<T>(f) <= (size_t)smem_bytes && f <= 32 * kSmallChunks) {
+    T* F = reinterpret_cast<T*>(smem_raw);
+    const int ld = small_ld(f);
+    int* iv = reinterpret_cast<int*>(F + small_entries<T>(f));
     for (int t = tid; t < 2 * f; t += BT) iv[t] = fvars[t];
-  assemble_front<T, BT>(d, node, F, f, ns, ndin, vals, rmap);
-  const int npiv = factor_front_rl<T, BT>(F, f, f, fs, fs == f, iv, iv + f,
-                                          ustab, pivot_tol, d.status, rs);
-  if (in_smem) {
-    for (size_t idx = tid; idx < (size_t)f * f; idx += BT) Fg[idx] = F[idx];
+    small_assemble<T, BT>(d, node, F, ld, f, ns, ndin, vals, iv + 4 * f);
+    int npiv = 0;
+    auto run = [&](auto chunks) {
+      npiv = small_factor<T, BT, decltype(chunks)::value>(F, f, fs, fs == f, iv, iv + f, ustab,
+                                                          pivot_tol, d.status, sc);
+    };
+    switch ((f + 31) / 32) {
+      case 1: run(std::integral_constant<int, 1>()); break;
+      case 2: run(std::integral_constant<int, 2>()); break;
+      case 3: run(std::integral_constant<int, 3>()); break;
+      case 4: run(std::integral_constant<int, 4>()); break;
+      default: run(std::integral_constant<int, kSmallChunks>());
+    }
+    const int lane = tid & 31;
+    for (int c = tid >> 5; c < f; c += BT / 32)
+      for (int r = c + lane; r < f; r += 32) Fg[r + (size_t)c * f] = F[r + (size_t)c * ld];
     for (int t = tid; t < 2 * f; t += BT) fvars[t] = iv[t];
     for (int t = tid; t < npiv; t += BT) fvars[3 * f + t] = iv[3 * f + t];
+    __syncthreads();
+    finish_front(d, node, F, ld, f, fs, npiv, fvars);
+  } else {
+    // scratch for the child row map: the front's W area
+    assemble_front<T, BT>(d, node, Fg, f, ns, ndin, vals,
+                          reinterpret_cast<int*>(Fg + (size_t)f * f));
+    const int npiv = factor_front_rl<T, BT>(Fg, f, f, fs, fs == f, fvars, fvars + f, ustab,
+                                            pivot_tol, d.status, rs);
+    __syncthreads();
+    finish_front(d, node, Fg, f, f, fs, npiv, fvars);
   }
-  __syncthreads();
-  finish_front(d, node, F, f, fs, npiv, fvars);
 }
 
 // ---------------------------------------------------------------------------
@@ -2660,7 +2679,6 @@ k_big_panel_cl(DevicePlan d, const int* __restrict__ nodes, double ustab,
   }
 }
 
-#include "pivot_fold.cuh"
 #include "panel_rows.cuh"
 
 template <class T>
@@ -2732,7 +2750,7 @@ k_big_finalize(DevicePlan d, const int* __restrict__ nodes) {
   const int f = d.f[node];
   const int fs = d.ns[node] + d.ndin[node];
   const int npiv = d.pstate[4 * node + 1];
-  finish_front(d, node, reinterpret_cast<const T*>(d.fpool) + d.foff[node], f,
+  finish_front(d, node, reinterpret_cast<const T*>(d.fpool) + d.foff[node], f, f,
                fs, npiv, d.ipool + d.ioff[node]);
 }
 
@@ -2902,7 +2920,7 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
   DevicePlan& d = h.d;
   static bool attr_set = false;
   if (!attr_set) {
-    FCUDA(cudaFuncSetAttribute(k_factor_level_rl<T, 256>,
+    FCUDA(cudaFuncSetAttribute(k_factor_level_rl<T, kRlThreads>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                kMaxDynSmem));
     FCUDA(cudaFuncSetAttribute(k_big_update<T>,
@@ -2992,7 +3010,7 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       // front + 5 int sections, sized for a few delayed pivots more than
       // the static front; larger fronts run in the pools
       const long long fm = L.small_max_f + kRlSlack;
-      long long bytes = ((fm * fm * (long long)sizeof(T) + 15) & ~15ll) + 5 * fm * 4;
+      long long bytes = (long long)small_bytes<T>((int)fm);
       if (bytes > kMaxDynSmem) bytes = kMaxDynSmem;
       k_factor_level_rl<T, kRlThreads><<<L.nsmall, kRlThreads, (size_t)bytes, s>>>(
           d, d.sched_nodes + L.small_begin, L.nsmall, d_vals, h.ustab,
