@@ -1299,6 +1299,13 @@ __device__ void assemble_front(const DevicePlan& d, int node, T* F, int f,
   }
 }
 
+// The kernels that begin a level are launched before the host has read whether
+// the level below is finished; where it is not they do nothing and are launched
+// again.
+__device__ __forceinline__ bool not_yet(const DevicePlan& d) {
+  return *((volatile int*)d.scratch_int) != 0;
+}
+
 #include "small_front.cuh"
 
 // Small fronts: the front and its four integer sections (variables,
@@ -1310,11 +1317,12 @@ template <class T, int BT>
 __global__ void __launch_bounds__(BT, 1024 / BT)
 k_factor_level_rl(DevicePlan d, const int* __restrict__ nodes, int count,
                   const double* __restrict__ vals, double ustab,
-                  double pivot_tol, int smem_bytes) {
+                  double pivot_tol, int smem_bytes, int below_big) {
   extern __shared__ double smem_raw[];
   __shared__ CtlT<BT> ctl;
   __shared__ RedSlots<BT> rs;
   __shared__ SmallCtl sc;
+  if (below_big && not_yet(d)) return;
   const int tid = threadIdx.x;
   const int node = nodes[blockIdx.x];
   if (!setup_front<T, BT>(d, node, ctl)) return;
@@ -1366,6 +1374,7 @@ k_factor_level_rl(DevicePlan d, const int* __restrict__ nodes, int count,
 template <class T>
 __global__ void __launch_bounds__(NT)
 k_big_setup(DevicePlan d, const int* __restrict__ nodes) {
+  if (not_yet(d)) return;
   __shared__ Ctl ctl;
   setup_front<T, NT>(d, nodes[blockIdx.x], ctl);
 }
@@ -1377,7 +1386,7 @@ __device__ __forceinline__ bool big_skip(const DevicePlan& d) {
 template <class T>
 __global__ void __launch_bounds__(NT)
 k_big_zero(DevicePlan d, const int* __restrict__ nodes) {
-  if (big_skip(d)) return;
+  if (big_skip(d) || not_yet(d)) return;
   const int node = nodes[blockIdx.x];
   const size_t f = d.f[node];
   T* F = reinterpret_cast<T*>(d.fpool) + d.foff[node];
@@ -1390,7 +1399,7 @@ template <class T>
 __global__ void __launch_bounds__(NT)
 k_big_add_A(DevicePlan d, const int* __restrict__ nodes,
             const double* __restrict__ vals) {
-  if (big_skip(d)) return;
+  if (big_skip(d) || not_yet(d)) return;
   const int node = nodes[blockIdx.x];
   const int f = d.f[node], ns = d.ns[node], ndin = d.ndin[node];
   T* F = reinterpret_cast<T*>(d.fpool) + d.foff[node];
@@ -1407,7 +1416,7 @@ k_big_add_A(DevicePlan d, const int* __restrict__ nodes,
 template <class T>
 __global__ void __launch_bounds__(NT)
 k_big_extend(DevicePlan d, const int* __restrict__ nodes, int q) {
-  if (big_skip(d)) return;
+  if (big_skip(d) || not_yet(d)) return;
   const int node = nodes[blockIdx.x];
   const int q0 = d.kid_ptr[node];
   if (q0 + q >= d.kid_ptr[node + 1]) return;
@@ -2742,30 +2751,66 @@ k_big_update_tc(DevicePlan d, const int* __restrict__ nodes) {
   tc::tc_end(c);
 }
 
+// Finishes the level's fronts that hold no more candidates, each once, and
+// counts the others; the last block to leave tells the host in scratch_int: how
+// many fronts are left (0 also when a pool ran out: the fronts stopped, the host
+// grows the pool and starts again; or a wait did: the host returns the error),
+// and the most rows and candidates of the next level's large fronts `up`, the
+// pivots that their children delayed included (what k_big_setup will find; not
+// used while fronts are left).  scratch_int: the answers 0 .. 2, blocks done 3,
+// fronts left so far 4.
 template <class T>
 __global__ void __launch_bounds__(NT)
-k_big_finalize(DevicePlan d, const int* __restrict__ nodes) {
-  if (big_skip(d)) return;
+k_big_finalize(DevicePlan d, const int* __restrict__ nodes, const int* __restrict__ up,
+               int nup) {
+  pdl_enter();
+  __shared__ int s_last, s_left, s_f, s_fs;
+  const int tid = threadIdx.x;
   const int node = nodes[blockIdx.x];
-  const int f = d.f[node];
-  const int fs = d.ns[node] + d.ndin[node];
-  const int npiv = d.pstate[4 * node + 1];
-  finish_front(d, node, reinterpret_cast<const T*>(d.fpool) + d.foff[node], f, f,
-               fs, npiv, d.ipool + d.ioff[node]);
-}
-
-// Number of large fronts of the level still holding candidates; 0 when a
-// pool ran out (the fronts stopped and the host grows the pool and
-// restarts the factorization) or a wait did (the host returns the error).
-__global__ void k_big_remaining(DevicePlan d, const int* __restrict__ nodes,
-                                int count, int* out) {
-  int r = 0;
-  for (int i = threadIdx.x; i < count; i += blockDim.x) {
-    const int* st = d.pstate + 4 * nodes[i];
-    r += st[0] < st[1] ? 1 : 0;
+  int* st = d.pstate + 4 * node;
+  const bool skip = big_skip(d);
+  if (!skip) {
+    const int k = st[0], npiv = st[1];
+    if (k < npiv) {
+      if (tid == 0) atomicAdd(d.scratch_int + 4, 1);
+    } else if (st[2] >= 0) {  // (-1: finished before)
+      const int f = d.f[node];
+      finish_front(d, node, reinterpret_cast<const T*>(d.fpool) + d.foff[node], f, f,
+                   d.ns[node] + d.ndin[node], npiv, d.ipool + d.ioff[node]);
+      if (tid == 0) st[2] = -1;
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
-  if (threadIdx.x == 0) *out = big_skip(d) ? 0 : r;
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(d.scratch_int + 3, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  if (tid == 0) {
+    __threadfence();
+    s_left = atomicExch(d.scratch_int + 4, 0);
+    d.scratch_int[3] = 0;
+    s_f = s_fs = 0;
+  }
+  __syncthreads();
+  // a warp per front, lanes over its children
+  for (int i = tid >> 5; i < nup && s_left == 0; i += NT / 32) {
+    const int p = up[i], lane = tid & 31;
+    int ndin = 0;
+    for (int q = d.kid_ptr[p] + lane; q < d.kid_ptr[p + 1]; q += 32)
+      ndin += __ldcg(d.ndel + d.kids[q]);
+    ndin = __reduce_add_sync(0xffffffffu, ndin);
+    if (lane == 0) {
+      atomicMax(&s_fs, d.ns[p] + ndin);
+      atomicMax(&s_f, d.ns[p] + ndin + d.nc[p]);
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    d.scratch_int[0] = skip ? 0 : s_left;
+    d.scratch_int[1] = s_f;
+    d.scratch_int[2] = s_fs;
+  }
 }
 
 }  // namespace
@@ -2984,6 +3029,11 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
   FCUDA(cudaMemsetAsync(d.counters, 0, 2 * sizeof(unsigned long long), s));
   FCUDA(cudaMemsetAsync(d.inertia, 0, 2 * sizeof(int) * d.nprob, s));
   FCUDA(cudaMemsetAsync(d.status, 0, sizeof(int), s));
+  FCUDA(cudaMemsetAsync(d.scratch_int, 0, 5 * sizeof(int), s));
+  if (!h.level_state) {
+    FCUDA(cudaHostAlloc((void**)&h.level_state, 3 * sizeof(int), cudaHostAllocDefault));
+    FCUDA(cudaEventCreateWithFlags(&h.level_event, cudaEventDisableTiming));
+  }
   // AMIGO_B200_TRACE=1 prints the device time of every level's small- and
   // large-front phases to stderr (diagnostics only).
   static const bool trace = std::getenv("AMIGO_B200_TRACE") != nullptr;
@@ -3003,7 +3053,8 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
     cudaMemsetAsync(dbg, 0, 64 * sizeof(int) * (size_t)d.num_levels, s);
     dbg_h.assign(64 * d.num_levels, 0);
   }
-  for (int l = 0; l < d.num_levels; l++) {
+  // Small fronts of a level, and its large fronts assembled.
+  auto begin_level = [&](int l) {
     const LevelSchedule& L = h.sched[l];
     if (trace) cudaEventRecord(ev[3 * l], s);
     if (L.nsmall) {
@@ -3014,12 +3065,11 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       if (bytes > kMaxDynSmem) bytes = kMaxDynSmem;
       k_factor_level_rl<T, kRlThreads><<<L.nsmall, kRlThreads, (size_t)bytes, s>>>(
           d, d.sched_nodes + L.small_begin, L.nsmall, d_vals, h.ustab,
-          h.pivot_tol, (int)bytes);
+          h.pivot_tol, (int)bytes, l > 0 && h.sched[l - 1].nbig > 0);
       ab::count_launch();
     }
     if (trace) cudaEventRecord(ev[3 * l + 1], s);
     if (L.nbig) {
-      int* dbg_l = dbg ? dbg + 64 * l : nullptr;
       const int* nodes = d.sched_nodes + L.big_begin;
       const int B = L.nbig;
       const long long fm = L.big_max_f;
@@ -3031,6 +3081,27 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       { k_big_add_A<T><<<dim3(B, std::max(ga, 1)), NT, 0, s>>>(d, nodes, d_vals); ab::count_launch(); }
       for (int q = 0; q < L.big_max_kids; q++)
         { k_big_extend<T><<<dim3(B, std::max(ge, 1)), NT, 0, s>>>(d, nodes, q); ab::count_launch(); }
+    }
+  };
+  // The level above large fronts begins while the host waits for their end, so
+  // its assembly hides the read; that read also returns the rows and candidates
+  // of its large fronts with the pivots their children delayed.  Otherwise the
+  // static sizes stand in, with room for kClSlack delays in the rows.
+  bool begun = false;
+  int next_rows = 0, next_fs = 0;  // 0: not known
+  for (int l = 0; l < d.num_levels; l++) {
+    const LevelSchedule& L = h.sched[l];
+    const int known_rows = next_rows, known_fs = next_fs;
+    next_rows = next_fs = 0;
+    if (!begun) begin_level(l);
+    begun = false;
+    if (L.nbig) {
+      int* dbg_l = dbg ? dbg + 64 * l : nullptr;
+      const int* nodes = d.sched_nodes + L.big_begin;
+      const int B = L.nbig;
+      const long long fm = L.big_max_f;
+      const int row_rows = known_rows ? std::max(known_rows, (int)fm) : (int)fm + kClSlack;
+      const long long max_fs = std::max(known_fs, L.big_max_fs);
       const long long ntl = (fm + kTile - 1) / kTile;
       int gu = (int)std::min<long long>(4 * 148, ntl * (ntl + 1) / 2);
       // shared-memory copy of the panel's L columns: as many rows as fit
@@ -3044,10 +3115,11 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       // shared-W panel for levels whose fronts fit its rows; its shared
       // memory holds up to NB columns of W for the largest static front
       // (fronts grown by delayed pivots get fewer columns)
-      // the row-per-thread panel (mode 0), for kClSlack rows more than the
-      // largest static front; in mode 2 the shared-memory cluster panel with
-      // the one-CTA panel's widths
-      const int row_rows = (int)fm + kClSlack;
+      // the row-per-thread panel (mode 0), for the level's rows: with the static
+      // size and a fixed slack, fronts that more delays had grown ran on one CTA
+      // from global memory (factorization of the 3D SIMP 20x10x10 KKT 47.3 ms
+      // then, 36.3 with the level's own, 12x6x6 in FP32 13.2 and 9.9); in mode 2 the shared-memory cluster panel
+      // with the one-CTA panel's widths
       const bool use_rows = h.panel_mode == 0 && fm >= h.cl_min_rows &&
                             row_rows <= (cl16_ok<T>() ? 32 : 8) * kRowThreads;
       const bool use_cl = h.panel_mode == 2 && fm >= h.cl_min_rows &&
@@ -3063,13 +3135,13 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       const bool force16 = h.panel_mode == 3 && cl16_ok<T>();
       const bool use_clg = ((h.panel_mode == 0 && !use_rows) ||
                             force16) &&
-                           fm >= h.cl_min_rows && fm + kClSlack <= gmax;
-      const bool g16 = use_clg && (force16 || fm + kClSlack > kClMaxRowsG8);
+                           fm >= h.cl_min_rows && row_rows <= gmax;
+      const bool g16 = use_clg && (force16 || row_rows > kClMaxRowsG8);
       long long g_stride = 0;
       if (use_clg) {
         const int gcs = g16 ? 16 : 8;
-        const long long glld = g16 ? cl_local_rows<16>((int)fm + kClSlack)
-                                   : cl_local_rows<8>((int)fm + kClSlack);
+        const long long glld = g16 ? cl_local_rows<16>(row_rows)
+                                   : cl_local_rows<8>(row_rows);
         g_stride = 2ll * NB * glld;
         const size_t need = (size_t)B * gcs * (size_t)g_stride * sizeof(T);
         if (need > h.cl_scratch_bytes) {
@@ -3094,7 +3166,7 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
         }
         panels += 2;
       } else {
-        panels = (int)((L.big_max_fs + NB - 2) / (NB - 1)) + 2;
+        panels = (int)((max_fs + NB - 2) / (NB - 1)) + 2;
       }
       // Every panel consumes at least one candidate of every unfinished
       // front, so no front needs more panels than it has rows.
@@ -3115,7 +3187,7 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
             if (rc) return rc;
           } else if (use_clg) {
             T* scr = reinterpret_cast<T*>(h.cl_scratch);
-            const int fr = (int)fm + kClSlack;
+            const int fr = row_rows;
             const int rc =
                 g16 ? launch_panel_cl<T, kClRowsG, 16, true>(B, 0, s, d, nodes, h.ustab,
                                                              h.pivot_tol, 0, fr, dbg_l, scr,
@@ -3158,23 +3230,34 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
             tupd[l] += b;
           }
         }
-        // Delayed pivots received from the children can make a front need
-        // more panels than its static size implies: check and continue.
-        { k_big_remaining<<<1, 32, 0, s>>>(d, nodes, B, d.scratch_int); ab::count_launch(); }
-        int left = 0;
-        FCUDA(cudaMemcpyAsync(&left, d.scratch_int, sizeof(int),
+        // Delayed pivots can make a front need more panels: the fronts that
+        // are done are finished, and the others go on.
+        const LevelSchedule* up = l + 1 < d.num_levels ? &h.sched[l + 1] : nullptr;
+        FCUDA(launch_pdl(k_big_finalize<T>, dim3(B), dim3(NT), (size_t)0, s, d, nodes,
+                         (const int*)(up ? d.sched_nodes + up->big_begin : nullptr),
+                         up ? up->nbig : 0));
+        ab::count_launch();
+        if (trace) cudaEventRecord(ev[3 * l + 2], s);
+        FCUDA(cudaMemcpyAsync(h.level_state, d.scratch_int, 3 * sizeof(int),
                               cudaMemcpyDeviceToHost, s));
-        FCUDA(cudaStreamSynchronize(s));
-        if (left == 0) break;
+        FCUDA(cudaEventRecord(h.level_event, s));
+        if (up) begin_level(l + 1);
+        FCUDA(cudaEventSynchronize(h.level_event));
+        if (h.level_state[0] == 0) {
+          begun = up != nullptr;
+          next_rows = h.level_state[1];
+          next_fs = h.level_state[2];
+          break;
+        }
         if (budget > max_panels) {
           std::fprintf(stderr, "amigo_b200: large-front panels did not finish\n");
           return -6;
         }
         panels = 4;
       }
-      { k_big_finalize<T><<<B, NT, 0, s>>>(d, nodes); ab::count_launch(); }
+    } else if (trace) {
+      cudaEventRecord(ev[3 * l + 2], s);
     }
-    if (trace) cudaEventRecord(ev[3 * l + 2], s);
   }
   if (trace) {
     cudaStreamSynchronize(s);

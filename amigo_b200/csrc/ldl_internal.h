@@ -132,6 +132,10 @@ struct LdlHandle {
   // global scratch of the cluster panel for fronts past shared memory
   void* cl_scratch = nullptr;
   size_t cl_scratch_bytes = 0;
+  // a level's end as the host reads it (pinned): large fronts left, the next
+  // level's rows and candidates
+  int* level_state = nullptr;
+  cudaEvent_t level_event = nullptr;
   long long wide_entries = 1 << 22;
   // front storage / arithmetic of the next factorization (64: FP64, 32:
   // FP32 fronts for mixed precision) and of the last one

@@ -205,7 +205,7 @@ int build_plan(LdlHandle& h, const int* rowp, const int* cols) {
   rc |= upload(&d.level_nodes, h.level_nodes);
   rc |= upload(&d.sched_nodes, sched_nodes);
   rc |= zalloc(&d.pstate, 4 * (size_t)nn);
-  rc |= zalloc(&d.scratch_int, 4);
+  rc |= zalloc(&d.scratch_int, 5);
   rc |= zalloc(&d.f, nn);
   rc |= zalloc(&d.npiv, nn);
   rc |= zalloc(&d.ndel, nn);
@@ -255,6 +255,12 @@ void free_plan(LdlHandle& h) {
   d = DevicePlan();
   h.cl_scratch = nullptr;
   h.cl_scratch_bytes = 0;
+  if (h.level_state) {
+    cudaFreeHost(h.level_state);
+    cudaEventDestroy(h.level_event);
+  }
+  h.level_state = nullptr;
+  h.level_event = nullptr;
   h.sv_bq = h.sv_dep = h.sv_err = nullptr;
   h.sv_done = h.sv_ctr = nullptr;
   h.sv_qlevels = h.sv_qcount = 0;
