@@ -136,7 +136,10 @@ struct LdlHandle {
   // level's rows and candidates
   int* level_state = nullptr;
   cudaEvent_t level_event = nullptr;
-  long long wide_entries = 1 << 22;
+  // fronts of this many f * npiv entries are solved by the whole grid: 3D SIMP
+  // 20x10x10 KKT 4.50 ms a solve (FP32 factor 4.83) against 4.54 (5.14) from
+  // 2^22 on, 4.82 (5.59) from 2^21 and 5.93 (5.83) never
+  long long wide_entries = 1 << 23;
   // front storage / arithmetic of the next factorization (64: FP64, 32:
   // FP32 fronts for mixed precision) and of the last one
   int precision = 64, factor_precision = 64;

@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <utility>
 #include <vector>
 
 #include "cluster_msg.cuh"
@@ -973,12 +974,26 @@ k_clu_backward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs,
 // since the last barrier are read with ld.global.cg (L2), never through
 // the non-coherent L1.  Sums run in a fixed order: the result does not
 // depend on the grid size.
+//
+// A step is a chain of latencies, not of bytes: the block's diagonal, its
+// triangle on one warp, two barriers and a share of the rows.  So the diagonal
+// block comes with 20 loads of a thread in flight, and the next one while the
+// others are at the rows; and a row's 128 terms are eight warps' partial sums
+// over 32-row strips, which occupy a CTA per strip.  One solve of the 3D SIMP
+// 20x10x10 KKT (a root of 3,925 pivots) takes 4.5 ms; 5.9 with the block
+// fetched at its turn entry by entry and one thread a row.
 constexpr int WB = 128;
 
 __device__ __forceinline__ int block_end_w(const int* kind, int jb, int npiv) {
   int je = jb + WB < npiv ? jb + WB : npiv;
   if (je < npiv && kind[je - 1] == 1) je++;
   return je;
+}
+
+__device__ __forceinline__ int block_begin_w(const int* kind, int je) {
+  int jb = je - WB > 0 ? je - WB : 0;
+  if (jb > 0 && kind[jb] == 2) jb--;  // keep 2x2 pairs together
+  return jb;
 }
 
 template <class T>
@@ -1014,6 +1029,33 @@ __device__ __forceinline__ long long first_item(long long base) {
   return r < 0 ? r + G : r;
 }
 
+// The lower triangle of the diagonal block of columns [jb, jb + bw) and its
+// pivot kinds into shared memory.
+template <class T>
+__device__ __forceinline__ void load_wide_block(const WideFront<T>& w, int jb, int bw,
+                                                double* sL, int* sK) {
+  constexpr int R = (WB + 32) / 32, C = 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int j0 = C * warp; j0 < bw; j0 += C * (NT / 32)) {
+    T a[C][R];
+#pragma unroll
+    for (int q = 0; q < C; q++)
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const int j = j0 + q, i = lane + 32 * r;
+        a[q][r] = j < bw && i >= j && i < bw ? w.L[jb + i + (size_t)(jb + j) * w.f] : T(0);
+      }
+#pragma unroll
+    for (int q = 0; q < C; q++)
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const int j = j0 + q, i = lane + 32 * r;
+        if (j < bw && i < bw) sL[i + j * (WB + 1)] = a[q][r];
+      }
+  }
+  for (int t = threadIdx.x; t < bw; t += NT) sK[t] = w.kind[jb + t];
+}
+
 template <class T>
 __global__ void __launch_bounds__(NT)
 k_wide_forward(DevicePlan d, const int* __restrict__ nodes, int count,
@@ -1026,6 +1068,7 @@ k_wide_forward(DevicePlan d, const int* __restrict__ nodes, int count,
   double* sv = sm + (WB + 1) * (WB + 1);   // WB + 1 block values
   __shared__ int sK[WB + 1];               // the block's pivot kinds
   __shared__ int s_choff;
+  __shared__ double part[NT / 32][32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int rhs = 0; rhs < nrhs; rhs++) {
     double* xr = x + (long long)rhs * ldx;
@@ -1038,25 +1081,25 @@ k_wide_forward(DevicePlan d, const int* __restrict__ nodes, int count,
       }
     }
     grid.sync();
+    // (a CTA with one front fetches its next block ahead)
+    const bool one = count <= (int)gridDim.x;
+    bool ahead = false;
+    int next = 0;  // where its front's next block begins (backward: ends)
     for (;;) {
       // sequential phase: next diagonal block of every front
       for (int c = blockIdx.x; c < count; c += gridDim.x) {
         const WideFront<T> w = wide_front<T>(d, nodes[c], ubuf, uoff, rhs);
         const int jb = __ldcg(wst + 2 * c + 1);
+        next = jb;
         if (jb >= w.npiv) {
           if (tid == 0) wst[2 * c] = jb;
           continue;
         }
         const int je = block_end_w(w.kind, jb, w.npiv);
         const int bw = je - jb;
-        for (int t = tid; t < bw * bw; t += NT) {
-          const int i = t % bw, j = t / bw;
-          sL[i + j * (WB + 1)] = w.L[jb + i + (size_t)(jb + j) * w.f];
-        }
-        for (int t = tid; t < bw; t += NT) {
-          sv[t] = __ldcg(w.G + jb + t);
-          sK[t] = w.kind[jb + t];
-        }
+        next = je;
+        if (!ahead) load_wide_block(w, jb, bw, sL, sK);
+        for (int t = tid; t < bw; t += NT) sv[t] = __ldcg(w.G + jb + t);
         __syncthreads();
         if (warp == 0) warp_lower_solve<(WB + 32) / 32>(sL, WB + 1, sK, bw, sv, lane);
         __syncthreads();
@@ -1067,7 +1110,16 @@ k_wide_forward(DevicePlan d, const int* __restrict__ nodes, int count,
         }
         __syncthreads();
       }
-      grid.sync();
+      auto token = grid.barrier_arrive();
+      ahead = false;
+      if (one && (int)blockIdx.x < count) {
+        const WideFront<T> w = wide_front<T>(d, nodes[blockIdx.x], ubuf, uoff, rhs);
+        if (next < w.npiv) {
+          load_wide_block(w, next, block_end_w(w.kind, next, w.npiv) - next, sL, sK);
+          ahead = true;
+        }
+      }
+      grid.barrier_wait(std::move(token));
       bool any = false;
       for (int c = 0; c < count && !any; c++)
         any = __ldcg(wst + 2 * c) < __ldcg(wst + 2 * c + 1);
@@ -1078,20 +1130,28 @@ k_wide_forward(DevicePlan d, const int* __restrict__ nodes, int count,
         const int jb = __ldcg(wst + 2 * c), je = __ldcg(wst + 2 * c + 1);
         if (jb >= je) continue;
         const WideFront<T> w = wide_front<T>(d, nodes[c], ubuf, uoff, rhs);
-        const long long items = (w.f - je + NT - 1) / NT;
+        const long long items = (w.f - je + 31) / 32;
         const int bw = je - jb;
+        const int q = (bw + NT / 32 - 1) / (NT / 32);  // terms of a warp
+        const int j0 = min(warp * q, bw), nj = min(q, bw - j0);
         bool staged = false;
         for (long long it = first_item(base); it < items; it += gridDim.x) {
+          __syncthreads();
           if (!staged) {
-            __syncthreads();
             for (int t = tid; t < bw; t += NT) sv[t] = __ldcg(w.G + jb + t);
             __syncthreads();
             staged = true;
           }
-          const int i = je + (int)it * NT + tid;
-          if (i < w.f) {
-            const double acc = dot_strided(w.L + i + (size_t)jb * w.f, (size_t)w.f, bw,
-                                           [&](int j) { return sv[j]; });
+          const int i = je + (int)it * 32 + lane;
+          part[warp][lane] =
+              i < w.f ? dot_strided(w.L + i + (size_t)(jb + j0) * w.f, (size_t)w.f, nj,
+                                    [&](int j) { return sv[j0 + j]; })
+                      : 0.0;
+          __syncthreads();
+          if (warp == 0 && i < w.f) {
+            double acc = part[0][lane];
+#pragma unroll
+            for (int p = 1; p < NT / 32; p++) acc = __dadd_rn(acc, part[p][lane]);
             w.G[i] = __ldcg(w.G + i) - acc;
           }
         }
@@ -1170,26 +1230,24 @@ k_wide_backward(DevicePlan d, const int* __restrict__ nodes, int count,
       }
     }
     grid.sync();
+    const bool one = count <= (int)gridDim.x;
+    bool ahead = false;
+    int next = 0;  // where its front's next block begins (backward: ends)
     for (;;) {
       // sequential phase: the next diagonal block from the end
       for (int c = blockIdx.x; c < count; c += gridDim.x) {
         const WideFront<T> w = wide_front<T>(d, nodes[c], ubuf, uoff, rhs);
         const int je = __ldcg(wst + 2 * c);
+        next = je;
         if (je <= 0) {
           if (tid == 0) wst[2 * c + 1] = je;
           continue;
         }
-        int jb = je - WB > 0 ? je - WB : 0;
-        if (jb > 0 && w.kind[jb] == 2) jb--;  // keep 2x2 pairs together
+        const int jb = block_begin_w(w.kind, je);
         const int bw = je - jb;
-        for (int t = tid; t < bw * bw; t += NT) {
-          const int i = t % bw, j = t / bw;
-          sL[i + j * (WB + 1)] = w.L[jb + i + (size_t)(jb + j) * w.f];
-        }
-        for (int t = tid; t < bw; t += NT) {
-          sv[t] = __ldcg(w.G + jb + t);
-          sK[t] = w.kind[jb + t];
-        }
+        next = jb;
+        if (!ahead) load_wide_block(w, jb, bw, sL, sK);
+        for (int t = tid; t < bw; t += NT) sv[t] = __ldcg(w.G + jb + t);
         __syncthreads();
         if (warp == 0) warp_upper_solve<(WB + 32) / 32>(sL, WB + 1, sK, bw, sv, lane);
         __syncthreads();
@@ -1200,7 +1258,17 @@ k_wide_backward(DevicePlan d, const int* __restrict__ nodes, int count,
         }
         __syncthreads();
       }
-      grid.sync();
+      auto token = grid.barrier_arrive();
+      ahead = false;
+      if (one && (int)blockIdx.x < count) {
+        const WideFront<T> w = wide_front<T>(d, nodes[blockIdx.x], ubuf, uoff, rhs);
+        if (next > 0) {
+          const int jb = block_begin_w(w.kind, next);
+          load_wide_block(w, jb, next - jb, sL, sK);
+          ahead = true;
+        }
+      }
+      grid.barrier_wait(std::move(token));
       bool any = false;
       for (int c = 0; c < count && !any; c++)
         any = __ldcg(wst + 2 * c) < __ldcg(wst + 2 * c + 1);
@@ -1502,7 +1570,7 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
   }
   if ((int)h.sv_fwd_grid.size() != d.num_levels || h.sv_grid_cap != wide_grid) {
     // Cooperative grids sized to the level's work (a grid-wide barrier
-    // costs more the more CTAs it spans): forward, one CTA per NT rows of
+    // costs more the more CTAs it spans): forward, one CTA per 32 rows of
     // the level's wide fronts; backward, one per 8 pivot columns (one warp
     // each); at least one per front, at most what is co-resident.
     h.sv_fwd_grid.assign(d.num_levels, 1);
@@ -1512,7 +1580,7 @@ static int launch_solve(LdlHandle& h, double* d_x, int nrhs, int ldx,
       const int wc = h.sv_narrow_ptr[l + 1] - h.sv_wide_ptr[l];
       for (int q = h.sv_wide_ptr[l]; q < h.sv_narrow_ptr[l + 1]; q++) {
         const int k = h.sv_host[q];
-        fr += (h.h_f[k] + NT - 1) / NT;
+        fr += (h.h_f[k] + 31) / 32;
         bc += (h.h_npiv[k] + 7) / 8;
       }
       h.sv_fwd_grid[l] = (int)std::min<long long>(wide_grid, std::max<long long>(fr, wc));

@@ -329,7 +329,7 @@ class SparseLDL:
 
     def set_wide_threshold(self, entries):
         """Fronts with f * npiv >= entries are solved by the multi-CTA
-        kernels (default 2^22)."""
+        kernels (default 2^23)."""
         _lib.call("ab_ldl_set_wide_threshold", self._h, int(entries))
 
     def stats(self):

@@ -126,7 +126,7 @@ int ab_ldl_set_tensor_cores(ab_ldl_t h, int on);
 int ab_ldl_set_panel_cache(ab_ldl_t h, int bytes);
 
 /* Solve schedule knobs: fronts with f * npiv >= the wide threshold
- * (default 2^22) are solved by the cooperative grid-wide kernels; fronts
+ * (default 2^23) are solved by the cooperative grid-wide kernels; fronts
  * from the cluster threshold (default 2^14) up to it by one thread-block
  * cluster of 8 CTAs each (when the front vector fits in shared memory);
  * smaller ones by one CTA per front.  All give the same result to
