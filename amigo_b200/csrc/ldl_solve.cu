@@ -1,6 +1,7 @@
 // Triangular solves with the multifrontal LDL^T factor (FP64).
 //
-// Forward sweep (levels ascending, one CTA per front): the front vector is
+// Forward sweep (levels ascending; a CTA, a cluster or the grid per front, by
+// size): the front vector is
 // assembled from the right-hand side of the node's own variables plus the
 // update vectors of its children, placed by the same row map as the
 // factorization's extend-add; L11 is applied in column blocks (one warp
