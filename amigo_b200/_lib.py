@@ -192,6 +192,7 @@ _SIGS = {
                                       ctypes.POINTER(IpmState), _vp, _vp, _vp,
                                       _vp, _vp, _vp, _vp, _vp]),
     "ab_launch_count": (ctypes.c_longlong, []),
+    "ab_ldl_set_wait_limit": (_i, [_vp, _i]),
     "ab_ldl_set_wide_threshold": (_i, [_vp, ctypes.c_longlong]),
     "ab_ldl_set_cluster_threshold": (_i, [_vp, ctypes.c_longlong]),
     "ab_ldl_set_panel_mode": (_i, [_vp, _i, _i]),

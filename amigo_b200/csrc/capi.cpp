@@ -466,6 +466,12 @@ int ab_ldl_set_panel_cache(ab_ldl_t h, int bytes) {
   return AB_OK;
 }
 
+int ab_ldl_set_wait_limit(ab_ldl_t h, int polls) {
+  if (!h || polls < 0) return AB_ERR_ARG;
+  h->h.d.wait_polls = polls;
+  return AB_OK;
+}
+
 int ab_ldl_set_wide_threshold(ab_ldl_t h, long long entries) {
   if (!h || entries < 1) return AB_ERR_ARG;
   h->h.wide_entries = entries;

@@ -1382,6 +1382,9 @@ k_big_setup(DevicePlan d, const int* __restrict__ nodes) {
   setup_front<T, NT>(d, nodes[blockIdx.x], ctl);
 }
 
+__device__ __forceinline__ bool pools_out(const DevicePlan& d) {
+  return (*((volatile int*)d.status) & (ST_POOL_F | ST_POOL_I)) != 0;
+}
 __device__ __forceinline__ bool big_skip(const DevicePlan& d) {
   return (*((volatile int*)d.status) & (ST_POOL_F | ST_POOL_I | ST_WAIT)) != 0;
 }

@@ -72,6 +72,7 @@ struct DevicePlan {
   int* status = nullptr;       // ST_* bits
   int* pstate = nullptr;       // per node: k, candidates left, kstart, kw
   int* scratch_int = nullptr;  // small device scratch for host queries
+  int wait_polls = 1 << 20;    // polls of a message's wait before it gives up
   unsigned long long* counters = nullptr;  // [F pool top, int pool top]
   double* fpool = nullptr;
   int* ipool = nullptr;

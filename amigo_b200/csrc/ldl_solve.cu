@@ -598,10 +598,11 @@ __device__ __forceinline__ void fetch_diag(const T* L, int f, int jb, int bw, do
 // the number of blocks.  forward: blocks from the first column on (block_end),
 // else from the last one backwards.
 __device__ __forceinline__ int clu_setup(const CluSmem& m, const int* kind, int npiv,
-                                         bool forward, int* s_nb) {
+                                         bool forward, int* s_nb, msg::Leave& leave) {
   const int tid = threadIdx.x;
   for (int j = tid; j < npiv; j += NT) m.K[j] = (unsigned char)kind[j];
   for (int b = tid; b < clu_blocks(npiv); b += NT) msg::init(m.bar + b);
+  msg::leave_init(leave);
   msg::init_done();
   __syncthreads();
   if (tid == 0) {
@@ -644,6 +645,7 @@ k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs, 
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double sm[];
   __shared__ int s_nb;
+  __shared__ msg::Leave s_leave;
   __shared__ int s_kid[kCluKids], s_cc[kCluKids];
   __shared__ long long s_uc[kCluKids];
   const int cr = (int)cluster.block_rank();
@@ -657,7 +659,7 @@ k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs, 
   const int ns = d.ns[node], ndin = d.ndin[node], fs = ns + ndin;
   const int* fsinv = fvars + 2 * f;
   const int q0 = d.kid_ptr[node], nk = d.kid_ptr[node + 1] - q0;
-  const int nb = clu_setup(m, fvars + 3 * f, npiv, true, &s_nb);
+  const int nb = clu_setup(m, fvars + 3 * f, npiv, true, &s_nb, s_leave);
   auto position = [&](int c, int ndc, int choff, int a) {
     int pos;
     if (a < ndc) {
@@ -795,7 +797,7 @@ k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs, 
 #pragma unroll
         for (int j = 0; j < SB; j++) a[j] = on && j < bw ? Li[(size_t)j * f] : T(0);
         const T a32 = on && bw > SB ? Li[(size_t)SB * f] : T(0);
-        msg::wait(m.bar + b, phase, err, kCluWait);
+        msg::wait(m.bar + b, phase, d.wait_polls, s_leave, err, kCluWait);
         int left = seg - jb % seg;  // columns to the end of the segment
         auto add = [&](double v, int j, double& s, double& acc, int& rest) {
           acc = __fma_rn(v, V[jb + j], acc);
@@ -851,6 +853,8 @@ k_clu_forward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs, 
     phase ^= 1u;
     cluster.sync();  // CTA 0's vector has been read
   }
+  if (__any_sync(0xffffffffu, *(volatile int*)&s_leave.dead))
+    msg::leave(&s_leave, err, kCluWait);
 }
 
 template <class T>
@@ -863,6 +867,7 @@ k_clu_backward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs,
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double sm[];
   __shared__ int s_nb;
+  __shared__ msg::Leave s_leave;
   const int cr = (int)cluster.block_rank();
   const int node = nodes[blockIdx.x / CS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -874,7 +879,7 @@ k_clu_backward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs,
   const CluSmem m = clu_smem(sm, f, npiv);
   double* V = m.V;            // CTA 0: pivot values, then the columns' corrections
   double* sx = m.V;           // the other CTAs: contribution rows' final values
-  const int nb = clu_setup(m, fvars + 3 * f, npiv, false, &s_nb);
+  const int nb = clu_setup(m, fvars + 3 * f, npiv, false, &s_nb, s_leave);
   double* cor = V + npiv;
   const bool rows = ncr > 0;
   if (cr == 0 && rows)
@@ -920,7 +925,7 @@ k_clu_backward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs,
       if (warp > 0 && nb > 0) load_pre(m.jb[1], m.jb[0]);
       for (int b = 0; b < nb; b++) {
         const int je = m.jb[b], jb = m.jb[b + 1];
-        if (rows) msg::wait(m.bar + b, phase, err, kCluWait);
+        if (rows) msg::wait(m.bar + b, phase, d.wait_polls, s_leave, err, kCluWait);
         cp_wait();
         __syncthreads();  // the last block's values
         // t[j] -= sum_{je <= i < npiv} L[i, j] t[i] for j in [jb, je)
@@ -962,6 +967,8 @@ k_clu_backward(DevicePlan d, const int* __restrict__ nodes, double* x, int nrhs,
     phase ^= 1u;
     cluster.sync();
   }
+  if (__any_sync(0xffffffffu, *(volatile int*)&s_leave.dead))
+    msg::leave(&s_leave, err, kCluWait);
 }
 
 // ---------------------------------------------------------------------------

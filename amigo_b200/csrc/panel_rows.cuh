@@ -51,6 +51,7 @@ struct RowCtl {
   // values of row k (its diagonal) and of row imax (diagonal, entry k)
   RowEntry we[2][2][NW];
   double ww[2][3];
+  msg::Leave leave;
   int kind[NB];
   int nm, nr;
   int mp[kRowMoves], mq[kRowMoves];             // moved positions and where their entries are
@@ -162,7 +163,8 @@ __host__ __device__ __forceinline__ size_t row_smem(int lld, int ncap) {
 template <class T, int PT, int RPT, int CS>
 __device__ void panel_factor_rows(T* F, int ld, T* Wg, int n, bool root, int* vars,
                                   int* fsperm, double ustab, double pivot_tol,
-                                  int* status, RowCtl<T, PT, CS>& c, T* Ws, int lld,
+                                  int* status, int polls,
+                                  RowCtl<T, PT, CS>& c, T* Ws, int lld,
                                   unsigned short* sl, unsigned short* ph,
                                   unsigned short* lst, int cr, int& k_, int& nc_,
                                   int& kw_) {
@@ -201,6 +203,7 @@ __device__ void panel_factor_rows(T* F, int ld, T* Wg, int n, bool root, int* va
   unsigned phase = 0;
   if constexpr (CS > 1) {
     if (tid < 8) msg::init(&c.bar[tid >> 2][tid & 3]);
+    msg::leave_init(c.leave);
     msg::init_done();
   }
   // every CTA of the cluster has started and its mbarriers are set up before
@@ -212,7 +215,7 @@ __device__ void panel_factor_rows(T* F, int ld, T* Wg, int n, bool root, int* va
     else {
       // (phase: the bits of the mbarriers' phases, one per mbarrier)
       const int bit = 4 * par + m;
-      msg::wait(&c.bar[par][m], (phase >> bit) & 1u, status, ST_WAIT);
+      msg::wait(&c.bar[par][m], (phase >> bit) & 1u, polls, c.leave, status, ST_WAIT);
       phase ^= 1u << bit;
     }
   };
@@ -570,6 +573,10 @@ __device__ void panel_factor_rows(T* F, int ld, T* Wg, int n, bool root, int* va
   // the panel's columns of F any more, L and D to F and W below the panel to
   // HBM, each CTA for its own rows
   row_barrier<CS>();
+  // (no CTA sends to another from here on)
+  if constexpr (CS > 1)
+    if (__any_sync(FULL, *(volatile int*)&c.leave.dead))
+      msg::leave(&c.leave, status, ST_WAIT);
   // D and W from shared memory, then L through it (each thread its own rows),
   // eight columns' loads before their stores
   constexpr int WB8 = 8 / RPT;
@@ -706,13 +713,18 @@ k_big_panel_rows(DevicePlan d, const int* __restrict__ nodes, double ustab,
   __shared__ RowCtl<T, PT, CS> c;
   __shared__ CtlT<PT> ctl;
   extern __shared__ double row_raw[];
-  if (big_skip(d)) return;
+  const bool skip = big_skip(d);
   int cr = 0;
   if constexpr (CS > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(cr));
   cr = row_uniform(cr);
   const int node = nodes[blockIdx.x / CS];
   int* st = d.pstate + 4 * node;
   int k = st[0], nc = st[1];
+  // (pools run out in earlier launches only; a wait, also in another cluster of
+  // this one, so that the CTAs of a cluster may read different answers: they
+  // start all the same, and those that know give up at their first wait)
+  const int over = __syncthreads_or(skip);
+  if (over && (CS == 1 || pools_out(d))) return;
   if (k >= nc) {
     if (cr == 0 && threadIdx.x == 0) st[3] = 0;
     return;
@@ -731,7 +743,8 @@ k_big_panel_rows(DevicePlan d, const int* __restrict__ nodes, double ustab,
     // (CTA 0 stores the state below only after the cluster's first barrier,
     // when every CTA has read it)
     panel_factor_rows<T, PT, RPT, CS>(F, f, W, f, fs == f, fvars, fvars + f, ustab,
-                                      pivot_tol, d.status, c, Ws, lld, sl, sl + ncap,
+                                      pivot_tol, d.status, over ? 0 : d.wait_polls, c, Ws, lld,
+                                      sl, sl + ncap,
                                       sl + 2 * ncap, cr, k, nc, kw);
   } else {
     row_barrier<CS>();

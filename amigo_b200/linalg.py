@@ -317,6 +317,12 @@ class SparseLDL:
         check (ab_ldl_solve_status)."""
         _lib.call("ab_ldl_solve_status", self._h, _stream_ptr(self.device))
 
+    def set_wait_limit(self, polls):
+        """Polls after which a wait for a message between the CTAs of a
+        front's cluster gives up (default 2^20): factor() raises then, and
+        solve_status() for a solve."""
+        _lib.call("ab_ldl_set_wait_limit", self._h, int(polls))
+
     def set_panel_mode(self, mode, min_rows=0):
         """Large-front panels: 0 (default) one row a thread on a thread-block
         cluster of 1 to 16 CTAs per front, on levels whose largest front has

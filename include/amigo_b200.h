@@ -125,6 +125,13 @@ int ab_ldl_set_tensor_cores(ab_ldl_t h, int on);
  * No reference counterpart. */
 int ab_ldl_set_panel_cache(ab_ldl_t h, int bytes);
 
+/* Polls after which a wait for a message between the CTAs of a front's
+ * cluster gives up (default 2^20; 0: at once, which a test of the error path
+ * uses).  A factorization whose wait ran out returns AB_ERR_CUDA and leaves the
+ * handle unfactored; a solve's is reported by ab_ldl_solve_status.  Either way
+ * the device stays usable.  No reference counterpart. */
+int ab_ldl_set_wait_limit(ab_ldl_t h, int polls);
+
 /* Solve schedule knobs: fronts with f * npiv >= the wide threshold
  * (default 2^23) are solved by the cooperative grid-wide kernels; fronts
  * from the cluster threshold (default 2^14) up to it by one thread-block
