@@ -1100,14 +1100,23 @@ __device__ int factor_front_rl(T* F, int ld, int n, int fs, bool root,
   return nc;
 }
 
+// A pool ran out; a pool or a wait did.
+__device__ __forceinline__ bool pools_out(const DevicePlan& d) {
+  return (*((volatile int*)d.status) & (ST_POOL_F | ST_POOL_I)) != 0;
+}
+__device__ __forceinline__ bool big_skip(const DevicePlan& d) {
+  return (*((volatile int*)d.status) & (ST_POOL_F | ST_POOL_I | ST_WAIT)) != 0;
+}
+
 // Front set-up shared by both paths (thread 0 sizes and allocates; all
 // threads fill the variable list and the fully-summed permutation record).
-// Returns false when the front must be skipped (a pool ran out earlier).
+// Returns false when the front must be skipped (a pool or a wait ran out
+// earlier: children that stopped have no pivot counts of this factorization).
 template <class T, int BT>
 __device__ bool setup_front(const DevicePlan& d, int node, CtlT<BT>& ctl) {
   const int tid = threadIdx.x;
   if (tid == 0) {
-    ctl.skip = (*((volatile int*)d.status) & (ST_POOL_F | ST_POOL_I)) ? 1 : 0;
+    ctl.skip = big_skip(d) ? 1 : 0;
     const int ns = d.ns[node], nc = d.nc[node];
     int ndin = 0;
     for (int q = d.kid_ptr[node]; q < d.kid_ptr[node + 1]; q++)
@@ -1382,12 +1391,6 @@ k_big_setup(DevicePlan d, const int* __restrict__ nodes) {
   setup_front<T, NT>(d, nodes[blockIdx.x], ctl);
 }
 
-__device__ __forceinline__ bool pools_out(const DevicePlan& d) {
-  return (*((volatile int*)d.status) & (ST_POOL_F | ST_POOL_I)) != 0;
-}
-__device__ __forceinline__ bool big_skip(const DevicePlan& d) {
-  return (*((volatile int*)d.status) & (ST_POOL_F | ST_POOL_I | ST_WAIT)) != 0;
-}
 
 template <class T>
 __global__ void __launch_bounds__(NT)

@@ -49,6 +49,24 @@ def test_panel_wait_runs_out(width, rows):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("width,rows", [(200, 60), (400, 5), (270, 100)])
+def test_small_front_above_a_wait_that_ran_out(width, rows, precision):
+    """The front above is one of the small ones, which are assembled from their
+    children's pivot counts: it is skipped (in a new handle the counts are 0,
+    and a child's rows would be more than the front has)."""
+    K = arrow(width, rows, 13, 0.4)
+    b = np.random.RandomState(3).randn(K.shape[0])
+    ldl, fresh = handle(K, precision), handle(K, precision)
+    ldl.set_wait_limit(0)
+    with pytest.raises(RuntimeError):
+        ldl.factor()
+    ldl.set_wait_limit(DEFAULT)
+    assert ldl.factor() == 0 and fresh.factor() == 0
+    assert ldl.get_inertia() == fresh.get_inertia()
+    assert np.array_equal(solution(ldl, b), solution(fresh, b))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
 @pytest.mark.parametrize("nrhs", [1, 17])
 def test_solve_wait_runs_out(precision, nrhs):
     K = arrow(180, 60, 12, 0.5)
