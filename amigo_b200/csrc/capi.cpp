@@ -171,11 +171,12 @@ int ab_ldl_mem_estimate(ab_ldl_t H, int precision, double delay_growth,
     csum += nc;
   }
   // front pool (in its element size, with room for delayed pivots), the
-  // int pool, the static plan (per-node arrays, contribution rows and their
+  // int pool, the static plan (27 ints a node, contribution rows and their
   // parent map, the assembly map of A: three ints per entry of the
-  // supernodes' columns, bounded by the fronts' fully-summed areas) and
-  // the solve's update vectors
-  long long plan = 64LL * (T.num_nodes + 1) + 8LL * csum + 4LL * T.n;
+  // supernodes' columns, bounded by the fronts' fully-summed areas), the
+  // solve's done flags and its update vectors
+  long long plan = (27LL + 2 * ab::kRhsSlices) * 4 * (T.num_nodes + 1) + 8LL * csum +
+                   4LL * T.n;
   long long amap = 0;
   for (int k = 0; k < T.num_nodes; k++) {
     const long long ns = T.node_ptr[k + 1] - T.node_ptr[k];
@@ -184,15 +185,29 @@ int ab_ldl_mem_estimate(ab_ldl_t H, int precision, double delay_growth,
   }
   plan += 12LL * amap;
   const long long solve = 8LL * fsum * (nrhs > 0 ? nrhs : 1);
-  // global scratch of the cluster panel for fronts past shared memory: W
-  // and L rows of NB columns for every CTA of a cluster of up to 16, with
-  // each CTA's rows rounded up to whole 32-row groups (bounded by the sum
-  // over those fronts)
-  long long clg = 0;
+  // global scratch of the panels of fronts past the row-per-thread panel, as
+  // large as the level that needs most of it: every large front of a level with
+  // such a front gets room for the level's rows, delayed pivots included
+  std::vector<int> level(T.num_nodes, 0);
+  std::vector<long long> rows, fronts_of;
   for (int k = 0; k < T.num_nodes; k++) {
+    for (int q = T.children_ptr[k]; q < T.children_ptr[k + 1]; q++)
+      level[k] = std::max(level[k], level[T.children[q]] + 1);
     const long long f = (T.node_ptr[k + 1] - T.node_ptr[k]) +
                         (T.contrib_ptr[k + 1] - T.contrib_ptr[k]);
-    if (f + 64 > 3072) clg += 2LL * ab::kPanel * (f + 64 + 16 * 32) * el;
+    if (!ab::large_front(f)) continue;
+    if ((int)rows.size() <= level[k]) {
+      rows.resize(level[k] + 1, 0);
+      fronts_of.resize(level[k] + 1, 0);
+    }
+    rows[level[k]] = std::max(rows[level[k]], f);
+    fronts_of[level[k]]++;
+  }
+  long long clg = 0;
+  for (size_t l = 0; l < rows.size(); l++) {
+    const long long r = std::max((long long)(g * (double)rows[l]), rows[l] + ab::kClSlack);
+    if (rows[l] && r > ab::kRowsMax16)
+      clg = std::max(clg, ab::panel_scratch(fronts_of[l], r, 16) * el);
   }
   *bytes = (long long)(g * (double)(fronts * el)) + (long long)(g * (double)(ints * 4)) +
            plan + solve + clg;

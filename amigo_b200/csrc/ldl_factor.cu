@@ -2065,7 +2065,6 @@ constexpr int kClCS = 8;
 // Rows a cluster panel takes: up to its threads' rows, capped so that W
 // and L of NB columns fit in a CTA's shared memory.
 constexpr int kClMaxRows = 3072;
-constexpr int kClSlack = 64;
 // Global-scratch cluster panel (GL): rows per thread; clusters of 8 take
 // fronts to 8 x 256 x 8 rows, of 16 to twice that.
 constexpr int kClRowsG = 8;
@@ -2701,6 +2700,7 @@ k_big_panel_cl(DevicePlan d, const int* __restrict__ nodes, double ustab,
 }
 
 #include "panel_rows.cuh"
+static_assert(kRowsMax16 == 32 * kRowThreads && kRowsMax8 == 8 * kRowThreads, "rows");
 
 template <class T>
 __global__ void __launch_bounds__(NT, 2)
@@ -3141,7 +3141,7 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       // then, 36.3 with the level's own, 12x6x6 in FP32 13.2 and 9.9); in mode 2 the shared-memory cluster panel
       // with the one-CTA panel's widths
       const bool use_rows = h.panel_mode == 0 && fm >= h.cl_min_rows &&
-                            row_rows <= (cl16_ok<T>() ? 32 : 8) * kRowThreads;
+                            row_rows <= (cl16_ok<T>() ? kRowsMax16 : kRowsMax8);
       const bool use_cl = h.panel_mode == 2 && fm >= h.cl_min_rows &&
                           fm + kClSlack <= kClMaxRows;
       const int cl_rule = h.panel_mode == 2 ? 1 : 0;
@@ -3160,10 +3160,8 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       long long g_stride = 0;
       if (use_clg) {
         const int gcs = g16 ? 16 : 8;
-        const long long glld = g16 ? cl_local_rows<16>(row_rows)
-                                   : cl_local_rows<8>(row_rows);
-        g_stride = 2ll * NB * glld;
-        const size_t need = (size_t)B * gcs * (size_t)g_stride * sizeof(T);
+        g_stride = panel_scratch(1, row_rows, gcs) / gcs;
+        const size_t need = (size_t)panel_scratch(B, row_rows, gcs) * sizeof(T);
         if (need > h.cl_scratch_bytes) {
           if (h.cl_scratch) FCUDA(cudaFree(h.cl_scratch));
           h.cl_scratch = nullptr;

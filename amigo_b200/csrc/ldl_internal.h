@@ -32,6 +32,29 @@ constexpr int kThreads = 256;
 // scheduled on that kernel when (f + 16)^2 + (f + 16) * kPanel doubles fit
 // (16 rows of slack for delayed pivots), otherwise on the multi-CTA path.
 constexpr int kMaxDynSmem = 190 * 1024;
+inline bool large_front(long long f) {
+  return ((f + 16) * (f + 16) + (f + 16) * kPanel) * 8 > kMaxDynSmem;
+}
+
+// Rows a level's large fronts are given beyond their static size where what
+// their children delayed is not known.
+constexpr int kClSlack = 64;
+// Rows up to which the row-per-thread panel takes a front, with clusters of 16
+// CTAs and without; past them a panel keeps W and L in global scratch.
+constexpr int kRowsMax16 = 8192, kRowsMax8 = 2048;
+// That scratch, in elements: W and L of kPanel columns for each CTA of a cluster
+// of cs, its rows in whole groups of 32, for each of a level's large fronts.
+inline long long panel_scratch(long long fronts, long long rows, int cs) {
+  return fronts * cs * 2 * kPanel * 32 * (((rows + 31) / 32 + cs - 1) / cs);
+}
+
+// Right-hand sides solved at the same time: slice y of a launch (blockIdx.y)
+// takes right-hand sides y, y + slices, ...; a front's chain of dependent steps
+// leaves most of the GPU idle, so the slices cost little more than one: eight
+// right-hand sides of the 3D 12x6x6 KKT 10.9 ms one after another, 1.27 ms so
+// (one alone 1.34 with FP32 fronts).  Each slice has its done
+// flags (a word per node and sweep).
+constexpr int kRhsSlices = 8;
 
 // Status bits written by device code.
 enum : int {

@@ -164,8 +164,7 @@ int build_plan(LdlHandle& h, const int* rowp, const int* cols) {
     for (int q = h.level_ptr[l]; q < h.level_ptr[l + 1]; q++) {
       const int k = h.level_nodes[q];
       const long long f = h.h_ns[k] + h.h_nc[k];
-      const long long fm = f + 16;
-      if ((fm * fm + fm * kPanel) * 8 <= kMaxDynSmem) {
+      if (!large_front(f)) {
         small.push_back(k);
         S.small_max_f = std::max<int>(S.small_max_f, (int)f);
       } else {

@@ -31,12 +31,6 @@ namespace {
 
 constexpr int NT = kThreads;
 constexpr int SB = 32;  // column block of the triangular solves
-// Right-hand sides solved at the same time: slice y of a launch (blockIdx.y)
-// takes right-hand sides y, y + slices, ...; a front's chain of dependent steps
-// leaves most of the GPU idle, so the slices cost little more than one: eight
-// right-hand sides of the 3D 12x6x6 KKT 10.9 ms one after another, 1.27 ms so
-// (one alone 1.34 with FP32 fronts).
-constexpr int kRhsSlices = 8;
 
 __device__ __forceinline__ int decode_var(int v) { return v >= 0 ? v : -v - 1; }
 
