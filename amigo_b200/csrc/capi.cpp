@@ -780,6 +780,20 @@ int ab_ldl_stats(ab_ldl_t H, void* stream, double* flops,
   return AB_OK;
 }
 
+int ab_ldl_panel_fallbacks(ab_ldl_t H, void* stream, int* count) {
+  if (!H || !count) return AB_ERR_ARG;
+  if (!H->h.factored) return AB_ERR_NOT_FACTORED;
+  if (!H->h.has_plan) return AB_ERR_UNSUPPORTED;
+  *count = 0;
+  if (H->h.sym.n == 0) return AB_OK;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (cudaMemcpyAsync(count, H->h.d.scratch_int + 5, sizeof(int), cudaMemcpyDeviceToHost,
+                      s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess)
+    return AB_ERR_CUDA;
+  return AB_OK;
+}
+
 int ab_ldl_node_pivots(ab_ldl_t H, void* stream, int* num_pivots,
                        int* num_delayed) {
   (void)stream;

@@ -2770,7 +2770,8 @@ k_big_update_tc(DevicePlan d, const int* __restrict__ nodes) {
 // and the most rows and candidates of the next level's large fronts `up`, the
 // pivots that their children delayed included (what k_big_setup will find; not
 // used while fronts are left).  scratch_int: the answers 0 .. 2, blocks done 3,
-// fronts left so far 4.
+// fronts left so far 4; 5 counts the panels of k_big_panel_rows that were too
+// large for their launch.
 template <class T>
 __global__ void __launch_bounds__(NT)
 k_big_finalize(DevicePlan d, const int* __restrict__ nodes, const int* __restrict__ up,
@@ -3041,7 +3042,7 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
   FCUDA(cudaMemsetAsync(d.counters, 0, 2 * sizeof(unsigned long long), s));
   FCUDA(cudaMemsetAsync(d.inertia, 0, 2 * sizeof(int) * d.nprob, s));
   FCUDA(cudaMemsetAsync(d.status, 0, sizeof(int), s));
-  FCUDA(cudaMemsetAsync(d.scratch_int, 0, 5 * sizeof(int), s));
+  FCUDA(cudaMemsetAsync(d.scratch_int, 0, 6 * sizeof(int), s));
   // (where there are large fronts: pinning takes longer than a small problem)
   bool large = false;
   for (const LevelSchedule& L : h.sched) large = large || L.nbig > 0;

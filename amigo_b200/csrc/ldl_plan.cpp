@@ -204,7 +204,7 @@ int build_plan(LdlHandle& h, const int* rowp, const int* cols) {
   rc |= upload(&d.level_nodes, h.level_nodes);
   rc |= upload(&d.sched_nodes, sched_nodes);
   rc |= zalloc(&d.pstate, 4 * (size_t)nn);
-  rc |= zalloc(&d.scratch_int, 5);
+  rc |= zalloc(&d.scratch_int, 6);
   rc |= zalloc(&d.f, nn);
   rc |= zalloc(&d.npiv, nn);
   rc |= zalloc(&d.ndel, nn);

@@ -749,6 +749,7 @@ k_big_panel_rows(DevicePlan d, const int* __restrict__ nodes, double ustab,
   } else {
     row_barrier<CS>();
     if (cr != 0) return;
+    if (threadIdx.x == 0) atomicAdd(d.scratch_int + 5, 1);
     panel_factor<T, PT>(F, f, W, f, f, fs == f, fvars, fvars + f, ustab, pivot_tol,
                         d.status, ctl, k, nc, kw);
   }

@@ -355,6 +355,14 @@ class SparseLDL:
                   _iptr(a), _iptr(b))
         return a, b
 
+    def panel_fallbacks(self):
+        """Panels of the last factorization (panel mode 0) whose front had more
+        rows than its level was launched for (ab_ldl_panel_fallbacks)."""
+        c = ctypes.c_int()
+        _lib.call("ab_ldl_panel_fallbacks", self._h, _stream_ptr(self.device),
+                  ctypes.byref(c))
+        return c.value
+
     def autotune(self, reps=3, cache=True):
         """Pick the large-front panel form and the solve schedule for this
         pattern by timing them on mat's current values

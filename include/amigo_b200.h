@@ -235,6 +235,12 @@ int ab_ldl_stats(ab_ldl_t h, void* stream, double* flops,
 int ab_ldl_node_pivots(ab_ldl_t h, void* stream, int* num_pivots,
                        int* num_delayed);
 
+/* Panels of the last factorization (panel mode 0) whose front had more rows
+ * than its level was launched for and which one CTA factored from global memory
+ * instead; 0 where the rows are known (synchronises).  No reference
+ * counterpart. */
+int ab_ldl_panel_fallbacks(ab_ldl_t h, void* stream, int* count);
+
 /* ----------------------------------------------------------------------
  * IPM vector kernels (include/interior_point_backend.h).  All array
  * arguments are device pointers; index arrays are int32.  The problem
