@@ -193,6 +193,7 @@ _SIGS = {
                                       ctypes.POINTER(IpmState), _vp, _vp, _vp,
                                       _vp, _vp, _vp, _vp, _vp]),
     "ab_launch_count": (ctypes.c_longlong, []),
+    "ab_ldl_set_general_forms": (_i, [_vp, _i]),
     "ab_ldl_set_wait_limit": (_i, [_vp, _i]),
     "ab_ldl_set_wide_threshold": (_i, [_vp, ctypes.c_longlong]),
     "ab_ldl_set_cluster_threshold": (_i, [_vp, ctypes.c_longlong]),

@@ -481,6 +481,12 @@ int ab_ldl_set_panel_cache(ab_ldl_t h, int bytes) {
   return AB_OK;
 }
 
+int ab_ldl_set_general_forms(ab_ldl_t h, int mask) {
+  if (!h || mask < 0 || mask > 3) return AB_ERR_ARG;
+  h->h.d.general_forms = mask;
+  return AB_OK;
+}
+
 int ab_ldl_set_wait_limit(ab_ldl_t h, int polls) {
   if (!h || polls < 0) return AB_ERR_ARG;
   h->h.d.wait_polls = polls;

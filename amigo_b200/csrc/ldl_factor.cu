@@ -1341,7 +1341,8 @@ k_factor_level_rl(DevicePlan d, const int* __restrict__ nodes, int count,
   const int f = ctl.f, fs = ctl.fs, ns = ctl.ns, ndin = ctl.ndin;
   int* fvars = d.ipool + ctl.ioff;
   T* Fg = pool + ctl.foff;
-  if (small_bytes<T>(f) <= (size_t)smem_bytes && f <= 32 * kSmallChunks) {
+  if (small_bytes<T>(f) <= (size_t)smem_bytes && f <= 32 * kSmallChunks &&
+      !(d.general_forms & 1)) {
     T* F = reinterpret_cast<T*>(smem_raw);
     const int ld = small_ld(f);
     int* iv = reinterpret_cast<int*>(F + small_entries<T>(f));

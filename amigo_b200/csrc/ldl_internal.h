@@ -96,6 +96,7 @@ struct DevicePlan {
   int* pstate = nullptr;       // per node: k, candidates left, kstart, kw
   int* scratch_int = nullptr;  // small device scratch for host queries
   int wait_polls = 1 << 20;    // polls of a message's wait before it gives up
+  int general_forms = 0;       // bit 0: small fronts, bit 1: narrow solves
   unsigned long long* counters = nullptr;  // [F pool top, int pool top]
   double* fpool = nullptr;
   int* ipool = nullptr;

@@ -316,6 +316,13 @@ __device__ void forward_front(const DevicePlan& d, int node, double* x, int nrhs
 
 #include "solve_front.cuh"
 
+// Whether a narrow front's pivot columns go to the launch's shared memory.
+template <class T>
+__device__ __forceinline__ bool solve_staged(const DevicePlan& d, int node, int smem_doubles) {
+  return staged_bytes<T>(d.f[node], d.npiv[node]) <= 8 * (size_t)smem_doubles &&
+         !(d.general_forms & 2);
+}
+
 template <class T, int NTH = NT>
 __global__ void __launch_bounds__(NTH)
 k_solve_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
@@ -325,7 +332,7 @@ k_solve_forward(DevicePlan d, const int* __restrict__ nodes, double* x,
   extern __shared__ double sV[];
   __shared__ NarrowSmem sm;
   const int node = nodes[blockIdx.x];
-  if (staged_bytes<T>(d.f[node], d.npiv[node]) <= 8 * (size_t)smem_doubles)
+  if (solve_staged<T>(d, node, smem_doubles))
     forward_staged<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, reinterpret_cast<char*>(sV),
                            []() {});
   else
@@ -392,7 +399,7 @@ k_solve_backward(DevicePlan d, const int* __restrict__ nodes, double* x,
   extern __shared__ double sV[];
   __shared__ NarrowSmem sm;
   const int node = nodes[blockIdx.x];
-  if (staged_bytes<T>(d.f[node], d.npiv[node]) <= 8 * (size_t)smem_doubles)
+  if (solve_staged<T>(d, node, smem_doubles))
     backward_staged<T, NTH>(d, node, x, nrhs, ldx, reinterpret_cast<char*>(sV), []() {});
   else
     backward_front<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, smem_doubles, sV, sm);
@@ -482,7 +489,7 @@ k_solve_forward_q(DevicePlan d, const int* __restrict__ nodes, int count, double
       for (int q = d.kid_ptr[node] + threadIdx.x; q < d.kid_ptr[node + 1]; q += NTH)
         wait_done(done + d.kids[q], epoch, err);
     };
-    if (staged_bytes<T>(d.f[node], d.npiv[node]) <= 8 * (size_t)smem_doubles) {
+    if (solve_staged<T>(d, node, smem_doubles)) {
       forward_staged<T, NTH>(d, node, x, nrhs, ldx, ubuf, uoff, reinterpret_cast<char*>(sV),
                              wait);
     } else {
@@ -514,7 +521,7 @@ k_solve_backward_q(DevicePlan d, const int* __restrict__ nodes,
     auto wait = [&]() {
       if (threadIdx.x == 0 && dep[idx] >= 0) wait_done(done + dep[idx], epoch, err);
     };
-    if (staged_bytes<T>(d.f[node], d.npiv[node]) <= 8 * (size_t)smem_doubles) {
+    if (solve_staged<T>(d, node, smem_doubles)) {
       backward_staged<T, NTH>(d, node, x, nrhs, ldx, reinterpret_cast<char*>(sV), wait);
     } else {
       wait();

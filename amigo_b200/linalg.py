@@ -317,6 +317,11 @@ class SparseLDL:
         check (ab_ldl_solve_status)."""
         _lib.call("ab_ldl_solve_status", self._h, _stream_ptr(self.device))
 
+    def set_general_forms(self, mask):
+        """Bit 0: small fronts factored, bit 1: narrow fronts solved, by the
+        general kernels (default 0; the same results bit for bit)."""
+        _lib.call("ab_ldl_set_general_forms", self._h, int(mask))
+
     def set_wait_limit(self, polls):
         """Polls after which a wait for a message between the CTAs of a
         front's cluster gives up (default 2^20): factor() raises then, and

@@ -125,6 +125,13 @@ int ab_ldl_set_tensor_cores(ab_ldl_t h, int on);
  * No reference counterpart. */
 int ab_ldl_set_panel_cache(ab_ldl_t h, int bytes);
 
+/* Forms of the small kernels, mask bits (default 0): bit 0 factors the small
+ * fronts with the general kernel on the pools, bit 1 solves the narrow ones with
+ * the general kernel that reads the factor from global memory, as fronts do that
+ * their shared memory does not hold.  The results are the same bit for bit (for
+ * tests).  No reference counterpart. */
+int ab_ldl_set_general_forms(ab_ldl_t h, int mask);
+
 /* Polls after which a wait for a message between the CTAs of a front's
  * cluster gives up (default 2^20; 0: at once, which a test of the error path
  * uses).  A factorization whose wait ran out returns AB_ERR_CUDA and leaves the
