@@ -2058,8 +2058,10 @@ k_big_panel_sw(DevicePlan d, const int* __restrict__ nodes, double ustab,
 //   * an interchange moves W rows between CTAs through distributed shared
 //     memory; F entries another CTA may have written in the same launch are
 //     read from L2.
-// With the one-CTA panel's widths (width_rule 1) the results are the one-
-// CTA panel's bit for bit; by default every panel takes NB columns.
+// Two forms: with W and L in shared memory (panel mode 2, a test mode) the
+// panels have the one-CTA panel's widths, and the results are its bit for bit;
+// with W and L in global scratch (GL: fronts past the row-per-thread panel, and
+// mode 3) every panel takes NB columns.
 constexpr int kClThreads = 256;
 constexpr int kClRows = 2;
 constexpr int kClCS = 8;
@@ -2612,8 +2614,8 @@ __host__ __device__ __forceinline__ int cl_local_rows(int cld) {
 template <class T, int PT, int RPT, int CS, bool TR, bool GL>
 __global__ void __launch_bounds__(PT, 1)
 k_big_panel_cl(DevicePlan d, const int* __restrict__ nodes, double ustab,
-               double pivot_tol, int smem_bytes, int width_rule, int fit_rows,
-               int* dbg, T* scratch, long long stride) {
+               double pivot_tol, int smem_bytes, int fit_rows, int* dbg, T* scratch,
+               long long stride) {
   pdl_enter();
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -2651,23 +2653,19 @@ k_big_panel_cl(DevicePlan d, const int* __restrict__ nodes, double ustab,
   int kw = 0;
   const int cld = f - kstart;
   const int lld = cl_local_rows<CS>(cld);
-  // the panel width depends on the front alone: NB, or the one-CTA
-  // panel's (width_rule 1)
+  // the panel width depends on the front alone: NB (GL), or the one-CTA
+  // panel's with its row limit, beyond which it takes the HBM-panel form, as
+  // below
   int nbe = NB;
-  int max_rows = GL ? CS * PT * RPT : kClMaxRows;
-  if (width_rule == 1) {
-    // the one-CTA panel's widths and its row limit (beyond which it takes
-    // the HBM-panel form, as below)
+  if (!GL) {
     const long long fit = (long long)kSwSmemBytes / ((long long)cld * (long long)sizeof(T));
     nbe = (int)(fit < NB ? fit : NB);
-    max_rows = kSwThreads * kSwRows;
   }
-  // full-width panels: fronts of up to fit_rows rows (the level's largest
-  // static front plus the slack its W and L rows were sized for, whatever
-  // the cluster size); the one-CTA widths: as long as W and L fit
-  const bool fits = width_rule == 0
-                        ? cld <= fit_rows
-                        : 2ll * nbe * lld * (long long)sizeof(T) <= smem_bytes;
+  const int max_rows = GL ? CS * PT * RPT : kSwThreads * kSwRows;
+  // GL: fronts of up to fit_rows rows (what the scratch was sized for, whatever
+  // the cluster size); else as long as W and L fit in shared memory
+  const bool fits = GL ? cld <= fit_rows
+                       : 2ll * nbe * lld * (long long)sizeof(T) <= smem_bytes;
   if (nbe >= 4 && cld <= max_rows && fits) {
     long long tk0 = 0;
     if (TR && dbg && cr == 0 && threadIdx.x == 0) {
@@ -2884,7 +2882,7 @@ static bool& cl16_ok() {
 template <class T, int RPT = kClRows, int CS = kClCS, bool GL = false>
 static int launch_panel_cl(int fronts, int smem, cudaStream_t s, const DevicePlan& d,
                            const int* nodes, double ustab, double pivot_tol,
-                           int width_rule, int fit_rows, int* dbg, T* scratch = nullptr,
+                           int fit_rows, int* dbg, T* scratch = nullptr,
                            long long stride = 0) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(fronts * CS);
@@ -2902,12 +2900,12 @@ static int launch_panel_cl(int fronts, int smem, cudaStream_t s, const DevicePla
   cfg.numAttrs = 2;
   if (dbg)
     FCUDA(cudaLaunchKernelEx(&cfg, k_big_panel_cl<T, kClThreads, RPT, CS, true, GL>, d,
-                             nodes, ustab, pivot_tol, smem, width_rule, fit_rows, dbg,
-                             scratch, stride));
+                             nodes, ustab, pivot_tol, smem, fit_rows, dbg, scratch,
+                             stride));
   else
     FCUDA(cudaLaunchKernelEx(&cfg, k_big_panel_cl<T, kClThreads, RPT, CS, false, GL>, d,
-                             nodes, ustab, pivot_tol, smem, width_rule, fit_rows,
-                             (int*)nullptr, scratch, stride));
+                             nodes, ustab, pivot_tol, smem, fit_rows, (int*)nullptr,
+                             scratch, stride));
   return 0;
 }
 
@@ -3134,19 +3132,15 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       const long long ntc = (fm + tc::TM - 1) / tc::TM;
       const int gtc = (int)std::max<long long>(
           1, std::min<long long>(3 * 148, ntc * (ntc + 1) / 2));
-      // shared-W panel for levels whose fronts fit its rows; its shared
-      // memory holds up to NB columns of W for the largest static front
-      // (fronts grown by delayed pivots get fewer columns)
       // the row-per-thread panel (mode 0), for the level's rows: with the static
       // size and a fixed slack, fronts that more delays had grown ran on one CTA
       // from global memory (factorization of the 3D SIMP 20x10x10 KKT 47.3 ms
-      // then, 36.3 with the level's own, 12x6x6 in FP32 13.2 and 9.9); in mode 2 the shared-memory cluster panel
-      // with the one-CTA panel's widths
+      // then, 36.3 with the level's own, 12x6x6 in FP32 13.2 and 9.9); in mode 2 the
+      // shared-memory cluster panel with the one-CTA panel's widths
       const bool use_rows = h.panel_mode == 0 && fm >= h.cl_min_rows &&
                             row_rows <= (cl16_ok<T>() ? kRowsMax16 : kRowsMax8);
       const bool use_cl = h.panel_mode == 2 && fm >= h.cl_min_rows &&
                           fm + kClSlack <= kClMaxRows;
-      const int cl_rule = h.panel_mode == 2 ? 1 : 0;
       const int cl_smem =
           use_cl ? 2 * NB * cl_local_rows<kClCS>((int)fm + kClSlack) * (int)sizeof(T) : 0;
       // past its rows: the cluster panel with its W and L rows in a global
@@ -3177,7 +3171,7 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       // panels a front of big_max_fs candidates needs without delays: each
       // takes nbe - 1 pivots, nbe growing as the remaining rows shrink
       int panels = 0;
-      if (use_sw || (use_cl && cl_rule == 1)) {
+      if (use_sw || use_cl) {
         for (long long kk = 0; kk < L.big_max_fs; panels++) {
           const long long rows = std::max<long long>(fm - kk, 1);
           const long long nbe = std::min<long long>(
@@ -3202,18 +3196,17 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
             if (rc) return rc;
           } else if (use_cl) {
             const int rc = launch_panel_cl<T>(B, cl_smem, s, d, nodes, h.ustab,
-                                              h.pivot_tol, cl_rule, (int)fm + kClSlack,
-                                              dbg_l);
+                                              h.pivot_tol, (int)fm + kClSlack, dbg_l);
             if (rc) return rc;
           } else if (use_clg) {
             T* scr = reinterpret_cast<T*>(h.cl_scratch);
             const int fr = row_rows;
             const int rc =
                 g16 ? launch_panel_cl<T, kClRowsG, 16, true>(B, 0, s, d, nodes, h.ustab,
-                                                             h.pivot_tol, 0, fr, dbg_l, scr,
+                                                             h.pivot_tol, fr, dbg_l, scr,
                                                              g_stride)
                     : launch_panel_cl<T, kClRowsG, 8, true>(B, 0, s, d, nodes, h.ustab,
-                                                            h.pivot_tol, 0, fr, dbg_l, scr,
+                                                            h.pivot_tol, fr, dbg_l, scr,
                                                             g_stride);
             if (rc) return rc;
           } else if (use_sw) {
