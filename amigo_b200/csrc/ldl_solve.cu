@@ -410,7 +410,6 @@ k_solve_backward(DevicePlan d, const int* __restrict__ nodes, double* x,
 // so the same bits).
 constexpr int kSmallRows = 128;
 constexpr int kSmallThreads = 128;
-constexpr int kSolveSms = 148;  // CTAs of a launch that run at once, one per SM
 
 // ---------------------------------------------------------------------------
 // Work-queue sweeps over the levels whose fronts are all narrow: one launch
@@ -1406,9 +1405,10 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
   // read the factor from global memory).  The cap leaves room for as many CTAs
   // per SM as the launch has fronts for, at most four: with more fronts than
   // that a front's latency is hidden by the others'.
+  int sms = 0;
+  SCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h.device));
   auto stage_cap = [&](int fronts) -> long long {
-    return fronts > 3 * kSolveSms ? 48 * 1024
-                                  : fronts > kSolveSms ? 96 * 1024 : kMaxDynSmem;
+    return fronts > 3 * sms ? 48 * 1024 : fronts > sms ? 96 * 1024 : kMaxDynSmem;
   };
   auto stage_bytes = [&](int k) -> long long {
     return (long long)(h.factor_precision == 32
