@@ -133,6 +133,7 @@ _SIGS = {
     "ab_ldl_stats": (_i, [_vp, _vp, _dp, _dp, _ip, _ip, _ip]),
     "ab_ldl_node_pivots": (_i, [_vp, _vp, _ip, _ip]),
     "ab_ldl_panel_fallbacks": (_i, [_vp, _vp, _ip]),
+    "ab_ldl_solve_plan": (_i, [_vp, ctypes.POINTER(ctypes.c_longlong)]),
     "ab_ldl_batch_create": (_i, [_i, _ip, ctypes.POINTER(_ip), ctypes.POINTER(_ip),
                                  _i, _i, _d, _d, _d, ctypes.POINTER(_vp)]),
     "ab_ldl_batch_inertia": (_i, [_vp, _vp, _ip, _ip]),

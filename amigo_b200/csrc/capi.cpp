@@ -786,6 +786,13 @@ int ab_ldl_stats(ab_ldl_t H, void* stream, double* flops,
   return AB_OK;
 }
 
+int ab_ldl_solve_plan(ab_ldl_t H, long long* count) {
+  if (!H || !count) return AB_ERR_ARG;
+  if (!H->h.factored) return AB_ERR_NOT_FACTORED;
+  *count = H->h.solve_plan + H->h.factor_epoch;
+  return AB_OK;
+}
+
 int ab_ldl_panel_fallbacks(ab_ldl_t H, void* stream, int* count) {
   if (!H || !count) return AB_ERR_ARG;
   if (!H->h.factored) return AB_ERR_NOT_FACTORED;

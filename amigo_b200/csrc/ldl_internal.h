@@ -198,6 +198,9 @@ struct LdlHandle {
   unsigned* sv_done = nullptr;   // forward, backward; per right-hand-side slice, node
   unsigned* sv_ctr = nullptr;    // forward, backward counters per slice; epoch
   int* sv_err = nullptr;
+  // changes of what a captured solve holds on to: the update vectors and their
+  // offsets, the fronts of each launch
+  long long solve_plan = 0;
 };
 
 int build_plan(LdlHandle& h, const int* rowp, const int* cols);

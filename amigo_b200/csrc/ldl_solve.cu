@@ -1375,6 +1375,7 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
     h.solve_epoch = h.factor_epoch;
     return 0;
   }
+  h.solve_plan++;
   std::vector<int>& nodes = h.sv_host;
   nodes.clear();
   nodes.reserve(nn);
@@ -1779,6 +1780,7 @@ int solve_numeric(LdlHandle& h, double* d_x, int nrhs, int ldx,
       (h.solve_epoch != h.factor_epoch && h.sv_f != h.h_f)) {
     // offsets of the update vectors (front sizes change with the delayed
     // pivots of each factorization)
+    h.solve_plan++;
     h.h_uoff.resize(nn);
     long long tot = 0;
     for (int k = 0; k < nn; k++) {

@@ -427,9 +427,11 @@ class SolveGraph:
     ``ldl.solve_device(xd)``, same bits) by replaying the graph on the
     current stream.  The solve's launch schedule depends on the front sizes
     of the factorization (delayed pivots), so the graph is captured again
-    on the first call after each ``ldl.factor()``; replays between
-    factorizations cost one graph launch instead of one launch per level
-    and sweep.  The work-queue sweeps take their epoch from device memory,
+    on the first call after each ``ldl.factor()``, and after a solve that
+    changed the handle's update vectors or schedule (another number of
+    right-hand sides, another threshold; ab_ldl_solve_plan); replays in
+    between cost one graph launch instead of one launch per level and
+    sweep.  The work-queue sweeps take their epoch from device memory,
     so every replay is a fresh sweep.  ``ab_launch_count`` counts the
     captured kernels once, at capture."""
 
@@ -439,9 +441,14 @@ class SolveGraph:
         self.ldl = ldl
         self.xd = xd
         self.graph = None
-        self._count = None
+        self._plan = None
         self.captures = 0
         self.replays = 0
+
+    def _solve_plan(self):
+        c = ctypes.c_longlong()
+        _lib.call("ab_ldl_solve_plan", self.ldl._h, ctypes.byref(c))
+        return c.value
 
     def _capture(self):
         ldl, xd = self.ldl, self.xd
@@ -455,11 +462,11 @@ class SolveGraph:
             with torch.cuda.graph(g):
                 ldl.solve_device(xd)
         self.graph = g
-        self._count = getattr(ldl, "factor_count", 0)
+        self._plan = self._solve_plan()
         self.captures += 1
 
     def __call__(self):
-        if self.graph is None or self._count != getattr(self.ldl, "factor_count", 0):
+        if self.graph is None or self._plan != self._solve_plan():
             self.graph = None
             self._capture()
         self.graph.replay()

@@ -242,6 +242,13 @@ int ab_ldl_stats(ab_ldl_t h, void* stream, double* flops,
 int ab_ldl_node_pivots(ab_ldl_t h, void* stream, int* num_pivots,
                        int* num_delayed);
 
+/* A count that changes with what a solve captured in a CUDA graph holds on to:
+ * the factorization, the number of right-hand sides of the last solve (its
+ * update vectors), the solve schedule.  Replay such a graph only while the
+ * count is what it was after the capture.  AB_ERR_NOT_FACTORED while the handle
+ * holds no factorization.  No reference counterpart. */
+int ab_ldl_solve_plan(ab_ldl_t h, long long* count);
+
 /* Panels of the last factorization (panel mode 0) whose front had more rows
  * than its level was launched for and which one CTA factored from global memory
  * instead; 0 where the rows are known (synchronises).  No reference
