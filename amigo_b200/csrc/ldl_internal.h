@@ -177,7 +177,7 @@ struct LdlHandle {
   std::vector<int> sv_narrow_ptr, sv_clu_ptr, sv_wide_ptr, sv_narrow_smem, sv_clu_smem;
   std::vector<int> sv_host, sv_f, sv_npiv;   // schedule and the sizes it is for
   int sv_max_wide = 0, sv_state_cap = 0;
-  long long sv_wide_entries = 0;
+  long long sv_wide_entries = 0, sv_cluster_entries = 0;
   std::vector<int> sv_fwd_grid, sv_bwd_grid;   // cooperative grid per level
   int sv_grid_cap = 0;
   // work-queue sweeps over the all-narrow levels [0, sv_qlevels): the

@@ -1371,7 +1371,8 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
   const int L = h.d.num_levels, nn = h.d.nn;
   // unchanged front sizes (the usual case between IPM iterations): keep it
   if (h.sv_f == h.h_f && h.sv_npiv == h.h_npiv && !h.sv_narrow_ptr.empty() &&
-      h.sv_wide_entries == h.wide_entries && h.sv_precision == h.factor_precision) {
+      h.sv_wide_entries == h.wide_entries && h.sv_cluster_entries == h.cluster_entries &&
+      h.sv_precision == h.factor_precision) {
     h.solve_epoch = h.factor_epoch;
     return 0;
   }
@@ -1519,6 +1520,7 @@ static int build_solve_schedule(LdlHandle& h, cudaStream_t s) {
   h.sv_npiv = h.h_npiv;
   h.sv_fwd_grid.clear();
   h.sv_wide_entries = h.wide_entries;
+  h.sv_cluster_entries = h.cluster_entries;
   h.sv_precision = h.factor_precision;
   h.solve_epoch = h.factor_epoch;
   return 0;
