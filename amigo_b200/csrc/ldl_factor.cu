@@ -3078,7 +3078,10 @@ static int launch_factor(LdlHandle& h, const double* d_vals, cudaStream_t s) {
       const long long fm = L.small_max_f + kRlSlack;
       long long bytes = (long long)small_bytes<T>((int)fm);
       if (bytes > kMaxDynSmem) bytes = kMaxDynSmem;
-      // (not by launch_pdl: 512 trajectories 5.57 ms a factorization, 5.75 with)
+      // (not by launch_pdl: it hides the drain of short levels, a direction of
+      // one trajectory 1.324 ms and 1.304 with, of 24 in FP32 3.47 and 3.43, but
+      // full levels, where the next CTAs take their slots early, lose more: 512
+      // trajectories 7.73 and 7.90, a factorization 5.57 and 5.75)
       k_factor_level_rl<T, kRlThreads><<<L.nsmall, kRlThreads, (size_t)bytes, s>>>(
           d, d.sched_nodes + L.small_begin, L.nsmall, d_vals, h.ustab,
           h.pivot_tol, (int)bytes, l > 0 && h.sched[l - 1].nbig > 0);

@@ -161,9 +161,15 @@ struct LdlHandle {
   // level's rows and candidates
   int* level_state = nullptr;
   cudaEvent_t level_event = nullptr;
-  // fronts of this many f * npiv entries are solved by the whole grid: 3D SIMP
-  // 20x10x10 KKT 4.50 ms a solve (FP32 factor 4.83) against 4.54 (5.14) from
-  // 2^22 on, 4.82 (5.59) from 2^21 and 5.93 (5.83) never
+  // fronts of this many f * npiv entries are solved by the whole grid: ms a
+  // solve of the 3D SIMP KKTs (FP32 factor), from 2^21 on, 2^22, 2^23 and never
+  //   20x10x10             4.77 (5.57)  4.48 (5.20)  4.44 (4.86)  5.44 (5.41)
+  //   16x8x8               2.39 (2.64)  2.39 (2.64)  2.39 (2.31)  2.39 (2.31)
+  //   20x10x10, 8 right-hand sides
+  //                        27.7 (32.4)  23.9 (27.8)  19.6 (22.7)  6.60 (6.75)
+  //   16x8x8, the same     12.5 (14.4)  12.5 (14.4)  3.16 (3.09)  3.16 (3.09)
+  // (one right-hand side decides here: the grid takes them one at a time, so
+  // several are faster with a higher threshold, ab_ldl_set_wide_threshold)
   long long wide_entries = 1 << 23;
   // front storage / arithmetic of the next factorization (64: FP64, 32:
   // FP32 fronts for mixed precision) and of the last one

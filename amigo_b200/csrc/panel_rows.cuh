@@ -26,8 +26,9 @@
 // as there: the results are the same bit for bit.  One factorization, before
 // (one-CTA panels to 768 rows, k_big_panel_cl above) and after: 2D SIMP 32x16
 // 4.57 -> 2.97 ms, 61x27 10.26 -> 5.94, 128x64 25.6 -> 16.9, 3D 20x10x10
-// 82.5 -> 46.8.  A step is bound by the latency of ~400 instructions of one
-// warp (ncu: 7 cycles from one to the next, no pipe above 30%).
+// 82.5 -> 46.8.  A step is bound by the latency of ~490 instructions of one
+// warp, the panel's end included (ncu, 1,120 rows on 8 CTAs: 8.8 cycles from one
+// to the next, no pipe above 20%).
 constexpr int kRowThreads = 256;
 
 constexpr int kRowMoves = 16;  // positions moved per flush

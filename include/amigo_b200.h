@@ -48,8 +48,9 @@ int ab_ldl_destroy(ab_ldl_t h);
 /* Device bytes a factorization of this pattern needs, from its symbolic
  * analysis alone (works on analysis-only handles, no GPU needed): the front
  * pool at `precision` (64 or 32) bits times delay_growth (room for fronts
- * grown by delayed pivots), the integer pools, the static plan and the
- * solve's update vectors for nrhs right-hand sides.  The admission budget
+ * grown by delayed pivots), the integer pools, the static plan, the solve's
+ * done flags and its update vectors for nrhs right-hand sides, and the global
+ * scratch of the panels of fronts past 8,192 rows.  The admission budget
  * of a request loop adds the caller's own vectors.  No counterpart call in
  * the reference, whose SparseLDL sizes its pools from the same symbolic
  * data (include/sparse_ldl.h:62-93, 3162-3220). */
@@ -175,8 +176,9 @@ int ab_ldl_set_panel_mode(ab_ldl_t h, int mode, int min_rows);
  *          256-thread ones (twice as many fronts in flight per SM;
  *          measured slower on the batched cart-pole and 2D SIMP KKTs).
  * All modes give the same result bit for bit.  ab_ldl_solve_status
- * reports (AB_ERR_CUDA) and clears a wait that ran out since the last
- * check; ab_ldl_factor also reports it.  No reference counterpart (the
+ * reports (AB_ERR_CUDA) and clears a wait of a solve (for a front of the
+ * queue, for a message of a cluster) that ran out since the last check;
+ * ab_ldl_factor also reports it.  No reference counterpart (the
  * reference solves front by front on the host). */
 int ab_ldl_set_solve_queue(ab_ldl_t h, int mode);
 int ab_ldl_solve_status(ab_ldl_t h, void* stream);
