@@ -93,8 +93,10 @@ __device__ __forceinline__ void store_to(int* p, int r, int v) {
 // that still run get on, to a wait that runs out in turn or to the end.  The
 // last warp takes part in the cluster's barriers until every CTA is down to its
 // last warp; no message is sent any more then, and the pause lets those under
-// way arrive.
-__device__ __forceinline__ void leave(Leave* e, int* status, int bit) {
+// way arrive.  (Out of line: it is long, and inlined at every wait it made the
+// kernels slower; eight right-hand sides of the 3D 12x6x6 KKT 2.493 ms, 2.473 so,
+// a direction of 2D SIMP 61x27 7.11 and 7.02.)
+static __device__ __noinline__ void leave(Leave* e, int* status, int bit) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   int cr, ncta;
